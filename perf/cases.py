@@ -45,7 +45,7 @@ def listed():
         # The plain mid benchmark workload: 256^3, CPML 12, scatterers inside a
         # plane wave's TF/SF box, 64 probes.
         dict(name="mid_scatterer", nx=256, ny=256, nz=256, layers=12, media="blocks", wave=True, probes=64, steps=8),
-        # The headline workload: 512^3 graded mesh, CPML 12, 30 % of the volume
+        # The headline workload: 512^3 graded mesh, CPML 12, a quarter of the volume
         # in two-pair pole-residue media, a dipole at the centre.
         dict(name="large_dispersive", nx=512, ny=512, nz=512, layers=12, media="dispersive", dipole=True, graded=True,
              probes=8, steps=2),
