@@ -613,12 +613,12 @@ sgpu_status launch_borders_h(sgpu_ctx* c) {
 }
 
 sgpu_status field_e(sgpu_ctx* c) {
-    if (c->family == 1 && tma_usable(c)) return launch_tma(c, false);
+    if (c->family == 1 && tma_usable(c)) return quads_usable(c) ? launch_quad(c, 0) : launch_tma(c, false);
     return c->cpml.on ? launch_e<kBulk | kCpml | kAll>(c) : launch_e<kBulk | kAll>(c);
 }
 
 sgpu_status field_h(sgpu_ctx* c) {
-    if (c->family == 1 && tma_usable(c)) return launch_tma(c, true);
+    if (c->family == 1 && tma_usable(c)) return quads_usable(c) ? launch_quad(c, 1) : launch_tma(c, true);
     return c->cpml.on ? launch_h<kBulk | kCpml | kAll>(c) : launch_h<kBulk | kAll>(c);
 }
 
@@ -851,6 +851,7 @@ void sgpu_destroy(sgpu_ctx* c) {
     free_list(c, c->probe_allocs);
     free_list(c, c->vprobe_allocs);
     free_farfields(c);
+    dev_free(c, c->quad_mem);
     if (c->stream && c->own_stream) cudaStreamDestroy(c->stream);
     if (c->host && c->host_free) c->host_free(c->host);
     delete c;
@@ -929,6 +930,7 @@ sgpu_status sgpu::set_media_tables(sgpu_ctx* c, int num_media, const float* g1, 
     }
     c->h_pec.assign(is_pec, is_pec + n1);
     c->num_media = num_media;
+    c->quad_ok = false;
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     return SGPU_OK;
 }
@@ -968,6 +970,8 @@ sgpu_status sgpu::narrow_media(sgpu_ctx* c, int comp) {
     return SGPU_OK;
 }
 
+void* sgpu::ctx_malloc(sgpu_ctx* c, size_t bytes) { return dev_malloc(c, bytes); }
+void sgpu::ctx_free(sgpu_ctx* c, void* p) { dev_free(c, p); }
 bool sgpu::tma_usable(const sgpu_ctx* c) { return c->tma_ready && c->num_media < 256; }
 void sgpu::keep_device_pool(int device) { keep_pool_memory(device); }
 
@@ -994,6 +998,7 @@ sgpu_status sgpu_download_field(sgpu_ctx* c, int comp, float* f) {
 sgpu_status sgpu_init_cpml(sgpu_ctx* c, const sgpu_cpml_desc* d) {
     if (!c || !d) return set_error(c, SGPU_ERR_ARG, "null cpml descriptor");
     free_list(c, c->cpml_allocs);
+    c->quad_ok = false;
     KCpml& k = c->cpml;
     k = KCpml{};
     sgpu_status s;
@@ -1936,6 +1941,7 @@ sgpu_status sgpu_advance_steps(sgpu_ctx* c, int n0, int count) {
     sgpu_status s = note_probe_rows(c, n0, count);
     if (s) return s;
     note_first_half(c, 2 * n0);
+    if (quads_usable(c) && (s = quad_prepare(c))) return s;
     const int chunk = std::min(count, 32);
     if (!c->graph || c->graph_steps != chunk) {
         if (c->graph) { cudaGraphExecDestroy(c->graph); c->graph = nullptr; }

@@ -301,6 +301,9 @@ struct sgpu_ctx {
     // graph
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
+    // tables of the quad kernels (quads.cu): one x table and two line tables a side
+    void* quad_mem = nullptr;
+    bool quad_ok = false;
     // scratch
     unsigned int* d_flag = nullptr;
     // TMA-pipelined fused kernels: tensor maps and the bounded-wait error word
@@ -330,6 +333,14 @@ sgpu_status create_in(const sgpu_grid_desc* d, Arena* arena, cudaStream_t stream
 // arena every probe keeps its whole trace (nsteps + 1 rows).
 sgpu_status host_create_in(const sgpu_problem* p, sgpu_ctx* plan, int max_steps, Arena* arena, cudaStream_t stream,
                            sgpu_ctx** out);
+// Device memory of a context (the batch's arena or the device's pool).
+void* ctx_malloc(sgpu_ctx* c, size_t bytes);
+void ctx_free(sgpu_ctx* c, void* p);
+// The curl + CPML half step of quads.cu (0 E, 1 H), its tables, and whether the
+// default kernel family takes it for this context.
+bool quads_usable(const sgpu_ctx* c);
+sgpu_status quad_prepare(sgpu_ctx* c);
+sgpu_status launch_quad(sgpu_ctx* c, int side);
 // UpdateFarField for every far field of the context (farfield.cu).
 sgpu_status launch_farfields(sgpu_ctx* c, StepRef sr);
 void free_farfields(sgpu_ctx* c);
