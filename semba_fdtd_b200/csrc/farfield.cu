@@ -42,6 +42,7 @@ struct FarArgs {
 
 __global__ void k_farfield_acc(KGrid g, FarArgs a, StepRef sr, int ox, int oy, int oz) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    grid_wait();
     if (q >= a.samples) return;
     const int n = step_of(sr);
     if ((n - 1) % a.ndecim) return;  // mod(ntime-1, Ndecim) /= 0 (Fortran MOD keeps the dividend's sign)
@@ -279,8 +280,7 @@ sgpu_status launch_farfields(sgpu_ctx* c, StepRef sr) {
     for (const FarField& F : c->farfields) {
         if (F.samples == 0) continue;
         const unsigned blocks = (unsigned)((F.samples + 255) / 256);
-        k_farfield_acc<<<blocks, 256, 0, c->stream>>>(kgrid(c), args_of(F), sr, c->ox, c->oy, c->oz);
-        const cudaError_t e = cudaGetLastError();
+        const cudaError_t e = launch_after(c->stream, blocks, 256, k_farfield_acc, kgrid(c), args_of(F), sr, c->ox, c->oy, c->oz);
         if (e != cudaSuccess) return set_error(c, SGPU_ERR_CUDA, std::string("k_farfield_acc: ") + cudaGetErrorString(e));
     }
     return SGPU_OK;

@@ -212,6 +212,7 @@ constexpr int kAdeBlock = 128;
 template <int NU, bool MAG, bool UNI>
 __global__ void __launch_bounds__(kAdeBlock, 12) k_ade(KGrid g, KDisp d, int comp) {
     const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    grid_wait();
     if (q < d.n[comp]) ade_node<NU, MAG, UNI>(ade_refs<MAG>(g, d, comp), q);
 }
 
@@ -219,19 +220,28 @@ __global__ void __launch_bounds__(kAdeBlock, 12) k_ade(KGrid g, KDisp d, int com
 // AdvancePlaneWaveE/H (planewaves.F90:878-1475) with Incid/evolucion
 // (:778-853) and AdvanceNodalE/H (nodalsources.F90:310-777): one thread per
 // touched node applies that node's contributions in the reference order.
+//
+// A row's contributions do not depend on the field, so they are formed before
+// grid_wait, beside the kernel before (the step counter, which they need, is
+// written two kernels back at the latest).  Most rows have one contribution;
+// the others keep their order by adding after the wait.
 __global__ void k_sources(KGrid g, KSrc s, StepRef sr, const double* tiempo, int t_n0, double dt, int hside, int mask) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = step_of(sr);
     const bool pw_on = (mask & (1 << kSrcPlaneWave)) ? pw_switch_block(s, n, tiempo, t_n0, dt, hside) : false;
     // with the switch down a row of plane-wave contributions alone changes
     // nothing: the reference calls no plane-wave routine then
-    if (s.pw_only && !pw_on) return;
-    if (r < s.nrows) source_row(g, s, n, tiempo, t_n0, dt, hside, mask, r, pw_on);
+    const bool live = r < s.nrows && !(s.pw_only && !pw_on);
+    SrcRow row{};
+    if (live) row = source_first(g, s, n, tiempo, t_n0, dt, hside, mask, r, pw_on);
+    grid_wait();
+    if (live) source_apply(s, row, mask, pw_on);
 }
 
 // UpdateObservation point probes (observation.F90:2633-2668).
 __global__ void k_probes(KGrid g, KProbes p, StepRef sr, int first_n) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    grid_wait();
     if (q < p.n) probe_one(g, p, step_of(sr), first_n, q);
 }
 
@@ -243,6 +253,7 @@ template <bool FREQ>
 __global__ void k_vol_probe(KGrid g, VolProbe p, StepRef sr, int ox, int oy, int oz) {
     const long long nodes = (long long)p.ni * p.nj * p.nk;
     const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    grid_wait();
     if (q >= nodes) return;
     const int n = step_of(sr);
     const int ii = (int)(q % p.ni), jj = (int)((q / p.ni) % p.nj), kk = (int)(q / ((long long)p.ni * p.nj));
@@ -273,9 +284,13 @@ __global__ void k_vol_probe(KGrid g, VolProbe p, StepRef sr, int ox, int oy, int
 // MinusCloneMagneticPMC / CloneMagneticPeriodic (bordersother.F90:65-190)
 // for the face kinds in `mask`, and AdvanceMagneticMUR (bordersmur.F90:502).
 __global__ void k_clone_h(KGrid g, KBorder b, int mask) {
+    grid_wait();
     clone_cell(g, b, mask, blockIdx.x * (long long)blockDim.x + threadIdx.x);
 }
-__global__ void k_mur_h(KGrid g, KBorder b) { mur_cell(g, b, blockIdx.x * (long long)blockDim.x + threadIdx.x); }
+__global__ void k_mur_h(KGrid g, KBorder b) {
+    grid_wait();
+    mur_cell(g, b, blockIdx.x * (long long)blockDim.x + threadIdx.x);
+}
 
 __global__ void k_fill_i16(int16_t* p, long long n, int v) {
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
@@ -509,8 +524,8 @@ sgpu_status build_sources(sgpu_ctx* c);
 
 template <int NU, bool MAG> void ade_launch(sgpu_ctx* c, int comp, unsigned blocks) {
     const KDisp& d = MAG ? c->mdisp : c->disp;
-    if (d.uniform && d.nu_max == NU) k_ade<NU, MAG, true><<<blocks, kAdeBlock, 0, c->stream>>>(kgrid(c), d, comp);
-    else k_ade<NU, MAG, false><<<blocks, kAdeBlock, 0, c->stream>>>(kgrid(c), d, comp);
+    if (d.uniform && d.nu_max == NU) launch_after(c->stream, blocks, kAdeBlock, k_ade<NU, MAG, true>, kgrid(c), d, comp);
+    else launch_after(c->stream, blocks, kAdeBlock, k_ade<NU, MAG, false>, kgrid(c), d, comp);
 }
 
 template <bool MAG> sgpu_status launch_ade_side(sgpu_ctx* c) {
@@ -559,7 +574,7 @@ sgpu_status launch_sources(sgpu_ctx* c, int side, StepRef sr, int mask = kMaskAl
         return set_error(c, SGPU_ERR_ARG, "step outside the time vector");
     int threads = 128;
     int blocks = (k.nrows + threads - 1) / threads;
-    k_sources<<<blocks, threads, 0, c->stream>>>(kgrid(c), k, sr, c->d_tiempo, c->t_n0, c->dt, side, mask);
+    launch_after(c->stream, blocks, threads, k_sources, kgrid(c), k, sr, c->d_tiempo, c->t_n0, c->dt, side, mask);
     return check_launch(c, "k_sources");
 }
 
@@ -571,15 +586,15 @@ sgpu_status launch_probes(sgpu_ctx* c, StepRef sr) {
     for (const VolProbe& p : c->vprobes) {
         const long long nodes = (long long)p.ni * p.nj * p.nk;
         const unsigned blocks = (unsigned)((nodes + 255) / 256);
-        if (p.kind == 0) k_vol_probe<true><<<blocks, 256, 0, c->stream>>>(kgrid(c), p, sr, c->ox, c->oy, c->oz);
-        else k_vol_probe<false><<<blocks, 256, 0, c->stream>>>(kgrid(c), p, sr, c->ox, c->oy, c->oz);
+        if (p.kind == 0) launch_after(c->stream, blocks, 256, k_vol_probe<true>, kgrid(c), p, sr, c->ox, c->oy, c->oz);
+        else launch_after(c->stream, blocks, 256, k_vol_probe<false>, kgrid(c), p, sr, c->ox, c->oy, c->oz);
         sgpu_status s = check_launch(c, "k_vol_probe");
         if (s) return s;
     }
     if (c->probes.n == 0) return SGPU_OK;
     int threads = 128;
     int blocks = (c->probes.n + threads - 1) / threads;
-    k_probes<<<blocks, threads, 0, c->stream>>>(kgrid(c), c->probes, sr, c->probe_first_n);
+    launch_after(c->stream, blocks, threads, k_probes, kgrid(c), c->probes, sr, c->probe_first_n);
     return check_launch(c, "k_probes");
 }
 
@@ -593,14 +608,14 @@ bool has_clone(const sgpu_ctx* c, int mask) {
 sgpu_status launch_clone(sgpu_ctx* c, int mask) {
     if (c->border.cl_cells == 0 || !has_clone(c, mask)) return SGPU_OK;
     const unsigned blocks = (unsigned)((c->border.cl_cells + 255) / 256);
-    k_clone_h<<<blocks, 256, 0, c->stream>>>(kgrid(c), c->border, mask);
+    launch_after(c->stream, blocks, 256, k_clone_h, kgrid(c), c->border, mask);
     return check_launch(c, "k_clone_h");
 }
 
 sgpu_status launch_mur(sgpu_ctx* c) {
     if (c->border.mur_cells == 0) return SGPU_OK;
     const unsigned blocks = (unsigned)((c->border.mur_cells + 255) / 256);
-    k_mur_h<<<blocks, 256, 0, c->stream>>>(kgrid(c), c->border);
+    launch_after(c->stream, blocks, 256, k_mur_h, kgrid(c), c->border);
     return check_launch(c, "k_mur_h");
 }
 

@@ -28,6 +28,8 @@ constexpr long long kQuadCells = 16ll << 20;
 template <int SIDE>
 __global__ void __launch_bounds__(kQuadThreads, 8)
     k_quad(const __grid_constant__ QuadView g, const __grid_constant__ QuadSide s, int chunk) {
+    // everything before grid_wait is constant over the run: it overlaps the
+    // kernel before
     __shared__ float2 tab[256];
     __shared__ QuadLine zl[kQuadChunk];
     for (int m = threadIdx.x; m < s.nmed1; m += kQuadThreads) tab[m] = s.tab[m];
@@ -47,6 +49,7 @@ __global__ void __launch_bounds__(kQuadThreads, 8)
     ld4(idx, X->id);
     const unsigned meet = valid ? X->meet & Y.hold : 0u, whole = X->whole;
     __syncthreads();
+    grid_wait();
     if (__any_sync(0xffffffffu, meet != 0)) quad_march<SIDE, true>(g, s, tab, zl, X, Y, idx, meet, whole, i, j, kb, ke, valid);
     else quad_march<SIDE, false>(g, s, tab, zl, X, Y, idx, meet, whole, i, j, kb, ke, valid);
 }
@@ -182,9 +185,8 @@ sgpu_status launch_quad(sgpu_ctx* c, int side) {
     while (chunk > 2 && (long long)bx * ((s.nz + chunk - 1) / chunk) < 148 * 16) chunk /= 2;
     const dim3 grid(bx, (s.nz + chunk - 1) / chunk);
     const QuadView v = quad_view(c);
-    if (side) k_quad<1><<<grid, kQuadThreads, 0, c->stream>>>(v, s, chunk);
-    else k_quad<0><<<grid, kQuadThreads, 0, c->stream>>>(v, s, chunk);
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = side ? launch_after(c->stream, grid, kQuadThreads, k_quad<1>, v, s, chunk)
+                               : launch_after(c->stream, grid, kQuadThreads, k_quad<0>, v, s, chunk);
     return e == cudaSuccess ? SGPU_OK : cuda_error(c, "k_quad", e);
 }
 

@@ -324,6 +324,32 @@ struct sgpu_ctx {
 };
 
 namespace sgpu {
+// Kernels of a step follow one another on a stream and each reads what the one
+// before wrote.  A kernel launched through launch_after may be scheduled while
+// its predecessor still runs: all its threads must call grid_wait (which
+// returns once the predecessor has finished and its writes are visible) before
+// they touch anything a kernel of the step writes, and before any of them
+// returns.  grid_wait also lets the kernel's own successor be scheduled.
+#ifdef __CUDACC__
+__device__ __forceinline__ void grid_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+cudaError_t launch_after(cudaStream_t stream, dim3 grid, int threads, void (*kernel)(P...), A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+#endif
+
 sgpu_status set_error(sgpu_ctx* c, sgpu_status code, const std::string& msg);
 KGrid kgrid(const sgpu_ctx* c);
 // sgpu_create with an optional arena and an external stream (batches).

@@ -550,37 +550,60 @@ __device__ __forceinline__ bool pw_switch_block(const KSrc& s, int n, const doub
 // (:778-853) and AdvanceNodalE/H (nodalsources.F90:310-777): source row r
 // (one touched node) applies that node's contributions in the reference
 // order; plane-wave contributions only while the global switch (pw_on) is up.
+//
+// A contribution adds w to the node (a soft one its negative) or, hard,
+// replaces it; kind 0: none.
+struct SrcTerm {
+    int kind;  // 0 none, 1 add, 2 replace
+    float w;
+};
+__device__ __forceinline__ SrcTerm source_term(const KSrc& s, const SrcEntry& en, float t, float G21, int mask, bool pw_on) {
+    if (!((1 << en.type) & mask)) return SrcTerm{0, 0.0f};
+    const SrcTable tb = s.tab[en.table];
+    const float* ev0 = s.samples + tb.offset;
+    float ev = 0.0f;
+    if (en.type == kSrcPlaneWave) {
+        if (!pw_on) return SrcTerm{0, 0.0f};
+        const long long nprev = (long long)((t - en.a) / tb.delta);
+        if (nprev + 1 <= tb.numus && nprev > 0)
+            ev = (ev0[nprev + 1] - ev0[nprev]) / tb.delta * ((t - en.a) - (float)nprev * tb.delta) + ev0[nprev];
+        const float inc = 0.0f + en.b * ev;
+        return SrcTerm{1, G21 * inc * en.c};
+    }
+    const long long nprev = (long long)(t / tb.delta);
+    if (!((nprev + 1 > tb.numus) || (nprev + 1 <= 0)))
+        ev = (ev0[nprev + 1] - ev0[nprev]) / tb.delta * ((t) - (float)nprev * tb.delta) + ev0[nprev];
+    return en.type == kSrcNodalSoft ? SrcTerm{1, -(en.a * ev)} : SrcTerm{2, en.a * ev};
+}
+__device__ __forceinline__ float source_add(float v, const SrcTerm& c) { return c.kind == 0 ? v : c.kind == 1 ? v + c.w : c.w; }
+
+struct SrcRow {
+    float* f;      // the node
+    float t, G21;  // time and coefficient of the half step
+    int p, end;    // contributions after the first
+    SrcTerm first;
+};
+__device__ __forceinline__ SrcRow source_first(const KGrid& g, const KSrc& s, int n, const double* tiempo, int t_n0, double dt,
+                                               int hside, int mask, int r, bool pw_on) {
+    SrcRow row;
+    const double tn = tiempo[n - t_n0];
+    row.t = hside ? (float)(tn + (double)0.5f * dt) : (float)tn;
+    row.G21 = hside ? g.gm2[1] : g.g2[1];
+    row.f = g.F[s.row_comp[r]] + s.row_node[r];
+    row.p = s.row_ptr[r];
+    row.end = s.row_ptr[r + 1];
+    row.first = source_term(s, s.e[row.p], row.t, row.G21, mask, pw_on);
+    ++row.p;
+    return row;
+}
+__device__ __forceinline__ void source_apply(const KSrc& s, const SrcRow& row, int mask, bool pw_on) {
+    float v = source_add(*row.f, row.first);
+    for (int p = row.p; p < row.end; ++p) v = source_add(v, source_term(s, s.e[p], row.t, row.G21, mask, pw_on));
+    *row.f = v;
+}
 __device__ __forceinline__ void source_row(const KGrid& g, const KSrc& s, int n, const double* tiempo, int t_n0, double dt,
                                            int hside, int mask, int r, bool pw_on) {
-    const double tn = tiempo[n - t_n0];
-    const float t = hside ? (float)(tn + (double)0.5f * dt) : (float)tn;
-    const float G21 = hside ? g.gm2[1] : g.g2[1];
-    float* F = g.F[s.row_comp[r]];
-    const int node = s.row_node[r];
-    float v = F[node];
-    for (int p = s.row_ptr[r]; p < s.row_ptr[r + 1]; ++p) {
-        const SrcEntry en = s.e[p];
-        if (!((1 << en.type) & mask)) continue;
-        const SrcTable tb = s.tab[en.table];
-        const float* ev0 = s.samples + tb.offset;
-        if (en.type == kSrcPlaneWave) {
-            if (!pw_on) continue;
-            float ev = 0.0f;
-            const long long nprev = (long long)((t - en.a) / tb.delta);
-            if (nprev + 1 <= tb.numus && nprev > 0)
-                ev = (ev0[nprev + 1] - ev0[nprev]) / tb.delta * ((t - en.a) - (float)nprev * tb.delta) + ev0[nprev];
-            const float inc = 0.0f + en.b * ev;
-            v = v + G21 * inc * en.c;
-        } else {
-            float ev = 0.0f;
-            const long long nprev = (long long)(t / tb.delta);
-            if (!((nprev + 1 > tb.numus) || (nprev + 1 <= 0)))
-                ev = (ev0[nprev + 1] - ev0[nprev]) / tb.delta * ((t) - (float)nprev * tb.delta) + ev0[nprev];
-            if (en.type == kSrcNodalSoft) v = v - en.a * ev;
-            else v = en.a * ev;
-        }
-    }
-    F[node] = v;
+    source_apply(s, source_first(g, s, n, tiempo, t_n0, dt, hside, mask, r, pw_on), mask, pw_on);
 }
 
 // UpdateObservation point probes (observation.F90:2633-2668).
