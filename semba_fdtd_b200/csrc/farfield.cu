@@ -22,53 +22,24 @@
 #include <complex>
 #include <vector>
 
+#include "observe.cuh"
 #include "sgpu_internal.h"
 #include "stencil.cuh"
 
 using namespace sgpu;
+using sgpu::dev::far_sample;
+using sgpu::dev::far_step;
 using sgpu::dev::step_of;
 
 namespace {
 
 constexpr float kPiF = 3.14159265358979323846f;  // pi of kind RKIND (fdetypes.F90:188)
 
-struct FarArgs {
-    FarPatch patch[kFarPatches];
-    int npatch, samples, nf, ndecim, w_m;
-    double2* acc;
-    const double2* wE;
-    const double2* wH;
-};
-
 __global__ void k_farfield_acc(KGrid g, FarArgs a, StepRef sr, int ox, int oy, int oz) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     grid_wait();
-    if (q >= a.samples) return;
-    const int n = step_of(sr);
-    if ((n - 1) % a.ndecim) return;  // mod(ntime-1, Ndecim) /= 0 (Fortran MOD keeps the dividend's sign)
-    // sampled steps before this one since step 0: the weight index
-    const int m = a.ndecim == 1 ? n : (n - 1) / a.ndecim;
-    if (m < 0 || m >= a.w_m) return;
-    int p = 0;
-    while (p + 1 < a.npatch && q >= a.patch[p + 1].off) ++p;
-    const FarPatch& P = a.patch[p];
-    const int r = q - P.off, w2 = P.hi2 - P.lo2 + 1;
-    const int o = P.lo1 + r / w2, u = P.lo2 + r % w2;
-    int i, j, k;
-    if (P.axis == 0) { i = P.plane; j = u; k = o; }
-    else if (P.axis == 1) { i = u; j = P.plane; k = o; }
-    else { i = u; j = o; k = P.plane; }
-    const long long c = (long long)(i - ox) + (long long)g.pitch * (j - oy) + g.plane * (long long)(k - oz);
-    const double v = (double)g.F[P.comp][c];
-    const double2* w = (P.comp >= 3 ? a.wH : a.wE) + (long long)m * a.nf;
-    for (int f = 0; f < a.nf; ++f) {
-        double2* s = a.acc + (long long)f * a.samples + q;
-        double2 x = *s;
-        const double2 wf = w[f];
-        x.x = x.x + wf.x * v;
-        x.y = x.y + wf.y * v;
-        *s = x;
-    }
+    int m;
+    if (q < a.samples && far_step(a, step_of(sr), m)) far_sample(g, a, m, 3, ox, oy, oz, q);
 }
 
 // One cell of the transform loops: the two E samples (t1 at position A, t2
@@ -238,19 +209,6 @@ __global__ void __launch_bounds__(kDirThreads) k_farfield_dir(const TCell* cells
 constexpr int kT[3][2] = {{2, 1}, {2, 0}, {1, 0}};
 inline int partner(int axis, int c) { return 3 + (3 - axis - c); }
 
-FarArgs args_of(const FarField& F) {
-    FarArgs a;
-    for (int p = 0; p < F.npatch; ++p) a.patch[p] = F.patch[p];
-    a.npatch = F.npatch;
-    a.samples = F.samples;
-    a.nf = F.nf;
-    a.ndecim = F.ndecim;
-    a.w_m = F.w_m;
-    a.acc = F.acc;
-    a.wE = F.wE;
-    a.wH = F.wH;
-    return a;
-}
 
 // complex(8) product as gfortran forms it (no fused operations)
 std::complex<double> cmul_h(std::complex<double> a, std::complex<double> b) {
@@ -276,11 +234,25 @@ float at(const std::vector<float>& v, int lo, int i) {
 
 namespace sgpu {
 
+FarArgs far_args(const FarField& F) {
+    FarArgs a;
+    for (int p = 0; p < F.npatch; ++p) a.patch[p] = F.patch[p];
+    a.npatch = F.npatch;
+    a.samples = F.samples;
+    a.nf = F.nf;
+    a.ndecim = F.ndecim;
+    a.w_m = F.w_m;
+    a.acc = F.acc;
+    a.wE = F.wE;
+    a.wH = F.wH;
+    return a;
+}
+
 sgpu_status launch_farfields(sgpu_ctx* c, StepRef sr) {
     for (const FarField& F : c->farfields) {
         if (F.samples == 0) continue;
         const unsigned blocks = (unsigned)((F.samples + 255) / 256);
-        const cudaError_t e = launch_after(c->stream, blocks, 256, k_farfield_acc, kgrid(c), args_of(F), sr, c->ox, c->oy, c->oz);
+        const cudaError_t e = launch_after(c->stream, blocks, 256, k_farfield_acc, kgrid(c), far_args(F), sr, c->ox, c->oy, c->oz);
         if (e != cudaSuccess) return set_error(c, SGPU_ERR_CUDA, std::string("k_farfield_acc: ") + cudaGetErrorString(e));
     }
     return SGPU_OK;

@@ -18,6 +18,7 @@
 #include <string>
 #include <vector>
 
+#include "observe.cuh"
 #include "sgpu_internal.h"
 #include "stencil.cuh"
 #include "tma_fields.cuh"
@@ -207,11 +208,19 @@ __global__ void __launch_bounds__(kTmaThreads, kTmaMinBlocks)
     else h_consume<0>(t, 0, g, cp, tab, err, false, rows[t.warp]);
 }
 
-// One node a thread, 128-thread blocks, 12 blocks an SM (40 registers).
+// One node a thread, 128-thread blocks, 12 blocks an SM (40 registers): one
+// component, or all three (blocks up to end0 the first's, up to end1 the
+// second's).
 constexpr int kAdeBlock = 128;
 template <int NU, bool MAG, bool UNI>
 __global__ void __launch_bounds__(kAdeBlock, 12) k_ade(KGrid g, KDisp d, int comp) {
     const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (q < d.n[comp]) ade_node<NU, MAG, UNI>(ade_refs<MAG>(g, d, comp), q);
+}
+template <int NU, bool MAG, bool UNI>
+__global__ void __launch_bounds__(kAdeBlock, 12) k_ade_all(KGrid g, KDisp d, int end0, int end1) {
+    const int b = blockIdx.x, comp = b < end0 ? 0 : b < end1 ? 1 : 2;
+    const long long q = (b - (comp == 0 ? 0 : comp == 1 ? end0 : end1)) * (long long)blockDim.x + threadIdx.x;
     grid_wait();
     if (q < d.n[comp]) ade_node<NU, MAG, UNI>(ade_refs<MAG>(g, d, comp), q);
 }
@@ -246,39 +255,12 @@ __global__ void k_probes(KGrid g, KProbes p, StepRef sr, int first_n) {
 }
 
 // Volume probes, one thread per sampled node (all three components).
-// FREQ: the frequency-domain accumulation of observation.F90:3527-3600,
-// V = V + w * F in complex(8) per frequency, component and node; else the
-// node's three values go into the frame of step n.
 template <bool FREQ>
 __global__ void k_vol_probe(KGrid g, VolProbe p, StepRef sr, int ox, int oy, int oz) {
     const long long nodes = (long long)p.ni * p.nj * p.nk;
     const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     grid_wait();
-    if (q >= nodes) return;
-    const int n = step_of(sr);
-    const int ii = (int)(q % p.ni), jj = (int)((q / p.ni) % p.nj), kk = (int)(q / ((long long)p.ni * p.nj));
-    const long long c = (long long)((p.i0 + ii) * p.tr[0] - ox) + (long long)g.pitch * ((p.j0 + jj) * p.tr[1] - oy) +
-                        g.plane * (long long)((p.k0 + kk) * p.tr[2] - oz);
-    const int f0 = p.magnetic ? 3 : 0;
-    const float v[3] = {g.F[f0][c], g.F[f0 + 1][c], g.F[f0 + 2][c]};
-    if (FREQ) {
-        const int m = n - p.w_n0;
-        if (m < 0 || m >= p.w_steps) return;
-        for (int f = 0; f < p.nf; ++f) {
-            const double2 w = p.w[(long long)m * p.nf + f];
-            for (int comp = 0; comp < 3; ++comp) {
-                double2* a = p.acc + (((long long)f * 3 + comp) * nodes + q);
-                double2 x = *a;
-                x.x = x.x + w.x * (double)v[comp];
-                x.y = x.y + w.y * (double)v[comp];
-                *a = x;
-            }
-        }
-    } else {
-        if (n < p.n_first || n >= p.n_last || (n - p.n_first) % p.every) return;
-        const long long slot = (long long)((n - p.n_first) / p.every) % p.cap;
-        for (int comp = 0; comp < 3; ++comp) p.ring[(slot * 3 + comp) * nodes + q] = v[comp];
-    }
+    if (q < nodes) vol_probe_node<FREQ>(g, p, step_of(sr), ox, oy, oz, nodes, q);
 }
 
 // MinusCloneMagneticPMC / CloneMagneticPeriodic (bordersother.F90:65-190)
@@ -522,30 +504,39 @@ bool ready(sgpu_ctx* c) {
 
 sgpu_status build_sources(sgpu_ctx* c);
 
-template <int NU, bool MAG> void ade_launch(sgpu_ctx* c, int comp, unsigned blocks) {
+// One launch for the three components, scheduled while its predecessor runs,
+// while they are a few waves of blocks; beyond, a plain launch each, so that
+// no waiting block takes a place from the one before (38 M nodes a component:
+// 7.46 ms for two steps, against 7.51 as one launch).
+constexpr long long kAdeTogether = 4ll << 20;
+template <int NU, bool MAG, bool UNI> void ade_launch(sgpu_ctx* c) {
     const KDisp& d = MAG ? c->mdisp : c->disp;
-    if (d.uniform && d.nu_max == NU) launch_after(c->stream, blocks, kAdeBlock, k_ade<NU, MAG, true>, kgrid(c), d, comp);
-    else launch_after(c->stream, blocks, kAdeBlock, k_ade<NU, MAG, false>, kgrid(c), d, comp);
+    int nb[3];
+    for (int comp = 0; comp < 3; ++comp) nb[comp] = (int)((d.n[comp] + kAdeBlock - 1) / kAdeBlock);
+    if (d.n[0] + d.n[1] + d.n[2] <= kAdeTogether) {
+        launch_after(c->stream, nb[0] + nb[1] + nb[2], kAdeBlock, k_ade_all<NU, MAG, UNI>, kgrid(c), d, nb[0], nb[0] + nb[1]);
+        return;
+    }
+    for (int comp = 0; comp < 3; ++comp)
+        if (nb[comp]) k_ade<NU, MAG, UNI><<<nb[comp], kAdeBlock, 0, c->stream>>>(kgrid(c), d, comp);
+}
+template <int NU, bool MAG> void ade_launch(sgpu_ctx* c) {
+    const KDisp& d = MAG ? c->mdisp : c->disp;
+    if (d.uniform && d.nu_max == NU) ade_launch<NU, MAG, true>(c);
+    else ade_launch<NU, MAG, false>(c);
 }
 
 template <bool MAG> sgpu_status launch_ade_side(sgpu_ctx* c) {
     const KDisp& d = MAG ? c->mdisp : c->disp;
     if (!(MAG ? c->mdisp_on : c->disp_on)) return SGPU_OK;
-    for (int comp = 0; comp < 3; ++comp) {
-        long long n = d.n[comp];
-        if (n == 0) continue;
-        const unsigned blocks = (unsigned)((n + kAdeBlock - 1) / kAdeBlock);
-        switch (d.nu_max) {
-            case 1: ade_launch<1, MAG>(c, comp, blocks); break;
-            case 2: ade_launch<2, MAG>(c, comp, blocks); break;
-            case 3: ade_launch<3, MAG>(c, comp, blocks); break;
-            case 4: ade_launch<4, MAG>(c, comp, blocks); break;
-            default: ade_launch<kMaxPolesPerMedium, MAG>(c, comp, blocks); break;
-        }
-        sgpu_status s = check_launch(c, "k_ade");
-        if (s) return s;
+    switch (d.nu_max) {
+        case 1: ade_launch<1, MAG>(c); break;
+        case 2: ade_launch<2, MAG>(c); break;
+        case 3: ade_launch<3, MAG>(c); break;
+        case 4: ade_launch<4, MAG>(c); break;
+        default: ade_launch<kMaxPolesPerMedium, MAG>(c); break;
     }
-    return SGPU_OK;
+    return check_launch(c, "k_ade");
 }
 
 sgpu_status launch_edisp(sgpu_ctx* c) { return launch_ade_side<false>(c); }
@@ -561,17 +552,25 @@ void note_first_half(sgpu_ctx* c, int h) {
     c->src[0].h_first = c->src[1].h_first = h;
 }
 
-sgpu_status launch_sources(sgpu_ctx* c, int side, StepRef sr, int mask = kMaskAll) {
+// The side's source lists, and the checks of a half step at a step the host knows.
+sgpu_status ready_sources(sgpu_ctx* c, int side, StepRef sr) {
     if (c->src_dirty) {
         sgpu_status s = build_sources(c);
         if (s) return s;
     }
     if (!sr.dev_n) note_first_half(c, 2 * sr.n + side);
-    const KSrc& k = c->src[side];
-    if (k.nrows == 0) return SGPU_OK;
+    if (c->src[side].nrows == 0) return SGPU_OK;
     if (!c->d_tiempo) return set_error(c, SGPU_ERR_STATE, "time vector not set (sgpu_set_time)");
     if (!sr.dev_n && (sr.n < c->t_n0 || sr.n >= c->t_n0 + c->d_tiempo_count))
         return set_error(c, SGPU_ERR_ARG, "step outside the time vector");
+    return SGPU_OK;
+}
+
+sgpu_status launch_sources(sgpu_ctx* c, int side, StepRef sr, int mask = kMaskAll) {
+    const sgpu_status st = ready_sources(c, side, sr);
+    if (st) return st;
+    const KSrc& k = c->src[side];
+    if (k.nrows == 0) return SGPU_OK;
     int threads = 128;
     int blocks = (k.nrows + threads - 1) / threads;
     launch_after(c->stream, blocks, threads, k_sources, kgrid(c), k, sr, c->d_tiempo, c->t_n0, c->dt, side, mask);
@@ -628,35 +627,58 @@ sgpu_status launch_borders_h(sgpu_ctx* c) {
 }
 
 sgpu_status field_e(sgpu_ctx* c) {
-    if (c->family == 1 && tma_usable(c)) return quads_usable(c) ? launch_quad(c, 0) : launch_tma(c, false);
+    if (c->family == 1 && tma_usable(c)) return quads_usable(c) ? launch_quad(c, 0, StepRef{nullptr, 0}, false, nullptr, nullptr) : launch_tma(c, false);
     return c->cpml.on ? launch_e<kBulk | kCpml | kAll>(c) : launch_e<kBulk | kAll>(c);
 }
 
 sgpu_status field_h(sgpu_ctx* c) {
-    if (c->family == 1 && tma_usable(c)) return quads_usable(c) ? launch_quad(c, 1) : launch_tma(c, true);
+    if (c->family == 1 && tma_usable(c)) return quads_usable(c) ? launch_quad(c, 1, StepRef{nullptr, 0}, false, nullptr, nullptr) : launch_tma(c, true);
     return c->cpml.on ? launch_h<kBulk | kCpml | kAll>(c) : launch_h<kBulk | kAll>(c);
 }
 
-sgpu_status half_e(sgpu_ctx* c, StepRef sr) {
-    sgpu_status s = field_e(c);
-    if (s) return s;
+// `obs`: the step whose observations of the other field ride in the half step
+// (quads.cu), or none.
+sgpu_status half_e(sgpu_ctx* c, StepRef sr, const StepRef* obs = nullptr) {
+    sgpu_status s;
+    bool sources = false;  // applied by the field kernel
+    if (c->family == 1 && quads_usable(c)) {
+        if ((s = ready_sources(c, 0, sr))) return s;
+        if ((s = launch_quad(c, 0, sr, !c->disp_on, obs, &sources))) return s;
+    } else if ((s = field_e(c))) {
+        return s;
+    }
     if ((s = launch_edisp(c))) return s;
-    return launch_sources(c, 0, sr);
+    return sources ? SGPU_OK : launch_sources(c, 0, sr);
 }
 
-sgpu_status half_h(sgpu_ctx* c, StepRef sr) {
-    sgpu_status s = field_h(c);
-    if (s) return s;
+sgpu_status half_h(sgpu_ctx* c, StepRef sr, const StepRef* obs = nullptr) {
+    sgpu_status s;
+    bool sources = false;
+    if (c->family == 1 && quads_usable(c)) {
+        if ((s = ready_sources(c, 1, sr))) return s;
+        if ((s = launch_quad(c, 1, sr, !c->mdisp_on, obs, &sources))) return s;
+    } else if ((s = field_h(c))) {
+        return s;
+    }
     if ((s = launch_mdisp(c))) return s;
-    if ((s = launch_sources(c, 1, sr))) return s;
+    if (!sources && (s = launch_sources(c, 1, sr))) return s;
     return launch_borders_h(c);
 }
 
-sgpu_status whole_step(sgpu_ctx* c, StepRef sr) {
-    sgpu_status s = half_e(c, sr);
-    if (s) return s;
-    if ((s = half_h(c, sr))) return s;
-    return launch_probes(c, sr);
+// `count` whole steps from sr.  Where the quad kernels run, the observations
+// that read E ride in the step's H half step (which leaves E alone) and those
+// that read H in the next step's E half step; the last step's follow it.
+sgpu_status whole_steps(sgpu_ctx* c, StepRef sr, int count) {
+    sgpu_status s = SGPU_OK;
+    const bool ride = c->family == 1 && quads_usable(c) && observers_ride(c);
+    for (int q = 0; q < count; ++q) {
+        const StepRef now{sr.dev_n, sr.n + q}, before{sr.dev_n, sr.n + q - 1};
+        if ((s = half_e(c, now, ride && q ? &before : nullptr))) return s;
+        if ((s = half_h(c, now, ride ? &now : nullptr))) return s;
+        if (!ride && (s = launch_probes(c, now))) return s;
+    }
+    if (ride && count > 0) return launch_observe(c, 1, StepRef{sr.dev_n, sr.n + count - 1});
+    return SGPU_OK;
 }
 
 // A context outside a batch takes its device memory from the device's
@@ -867,6 +889,7 @@ void sgpu_destroy(sgpu_ctx* c) {
     free_list(c, c->vprobe_allocs);
     free_farfields(c);
     dev_free(c, c->quad_mem);
+    free_list(c, c->quad_src_allocs);
     if (c->stream && c->own_stream) cudaStreamDestroy(c->stream);
     if (c->host && c->host_free) c->host_free(c->host);
     delete c;
@@ -1317,9 +1340,15 @@ long long lin(const sgpu_ctx* c, int i, int j, int k) {
 }
 
 sgpu_status build_sources(sgpu_ctx* c) {
+    c->quad_src_ok = false;
+    if (c->graph) {  // captured launches hold the old lists
+        cudaGraphExecDestroy(c->graph);
+        c->graph = nullptr;
+    }
     for (int side = 0; side < 2; ++side) {
         free_list(c, c->src_allocs[side]);
         c->src[side] = KSrc{};
+        c->src_rows[side] = SrcRows{};
         const std::vector<sgpu_ctx::HostEntry>& es = c->src_host[side];
         if (es.empty()) continue;
         if (es.size() >= (1u << 30)) return set_error(c, SGPU_ERR_UNSUPPORTED, "too many source contributions");
@@ -1385,6 +1414,14 @@ sgpu_status build_sources(sgpu_ctx* c) {
         k.h_first = c->h_first;
         k.pw_only = 1;
         for (const SrcEntry& en : ent) k.pw_only &= en.type == kSrcPlaneWave;
+        if (!c->arena && quads_usable(c) && rows_ride(c, side)) {
+            SrcRows& h = c->src_rows[side];
+            h.first.reserve(rnode.size());
+            for (size_t r = 0; r < rnode.size(); ++r) h.first.push_back(ent[rptr[r]]);
+            h.node = std::move(rnode);
+            h.comp = std::move(rcomp);
+            h.ptr = std::move(rptr);
+        }
     }
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     c->src_dirty = false;
@@ -1956,14 +1993,14 @@ sgpu_status sgpu_advance_steps(sgpu_ctx* c, int n0, int count) {
     sgpu_status s = note_probe_rows(c, n0, count);
     if (s) return s;
     note_first_half(c, 2 * n0);
-    if (quads_usable(c) && (s = quad_prepare(c))) return s;
+    if (quads_usable(c) && (s = quad_ready(c))) return s;
     const int chunk = std::min(count, 32);
     if (!c->graph || c->graph_steps != chunk) {
         if (c->graph) { cudaGraphExecDestroy(c->graph); c->graph = nullptr; }
         cudaGraph_t g;
         CUDA_TRY(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
         sgpu_status cs = SGPU_OK;
-        for (int q = 0; q < chunk && !cs; ++q) cs = whole_step(c, StepRef{c->d_step, q});
+        cs = whole_steps(c, StepRef{c->d_step, 0}, chunk);
         if (!cs) {
             k_add_step<<<1, 1, 0, c->stream>>>(c->d_step, chunk);
             cs = check_launch(c, "k_add_step");
@@ -1983,8 +2020,7 @@ sgpu_status sgpu_advance_steps(sgpu_ctx* c, int n0, int count) {
         CUDA_TRY(c, cudaGraphLaunch(c->graph, c->stream));
         done += chunk;
     }
-    for (; done < count; ++done)
-        if ((s = whole_step(c, StepRef{nullptr, n0 + done}))) return s;
+    if ((s = whole_steps(c, StepRef{nullptr, n0 + done}, count - done))) return s;
     if (c->probes.n) c->probe_written += count;
     c->steps_hi = std::max(c->steps_hi, n0 + count);
     return SGPU_OK;
@@ -2142,12 +2178,12 @@ sgpu_status sgpu_select_device(int device) {
 sgpu_status sgpu_kernels_per_step(const sgpu_ctx* c, int* n) {
     if (!c || !n) return SGPU_ERR_ARG;
     int k = 2;  // E and H field kernels
-    for (int comp = 0; comp < 3; ++comp) k += c->disp_on && c->disp.n[comp] > 0;
-    for (int comp = 0; comp < 3; ++comp) k += c->mdisp_on && c->mdisp.n[comp] > 0;
-    k += c->src[0].nrows > 0;
-    k += c->src[1].nrows > 0;
-    k += c->probes.n > 0;
-    k += (int)c->vprobes.size();
+    const bool quads = c->family == 1 && quads_usable(c), ride = quads && observers_ride(c);
+    for (const KDisp* d : {c->disp_on ? &c->disp : nullptr, c->mdisp_on ? &c->mdisp : nullptr})
+        if (d) k += d->n[0] + d->n[1] + d->n[2] <= kAdeTogether ? 1 : (d->n[0] > 0) + (d->n[1] > 0) + (d->n[2] > 0);
+    k += c->src[0].nrows > 0 && !(quads && !c->disp_on && c->quad_src_fits && rows_ride(c, 0));
+    k += c->src[1].nrows > 0 && !(quads && !c->mdisp_on && c->quad_src_fits && rows_ride(c, 1));
+    if (!ride) k += (c->probes.n > 0) + (int)c->vprobes.size();
     k += c->border.cl_cells > 0;
     k += c->border.mur_cells > 0;
     *n = k;

@@ -3,8 +3,10 @@
 
 #include <algorithm>
 #include <string>
+#include <type_traits>
 #include <vector>
 
+#include "observe.cuh"
 #include "quads.cuh"
 #include "sgpu_internal.h"
 
@@ -25,24 +27,136 @@ constexpr int kQuadChunk = 4;
 // taking turns: 395 / 353..387.
 constexpr long long kQuadCells = 16ll << 20;
 
+constexpr int kQuadVol = 4;  // volume probes the arguments hold
+
+// A source row with its first contribution beside it.
+struct QuadRow {
+    int node, comp, count, first;
+    SrcEntry e;
+};
+// The source rows of a half step by (warp's quads, plane), and what a row needs.
+struct QuadSrc {
+    const int* ptr;  // null: none
+    const QuadRow* row;
+    KSrc s;
+    const double* tiempo;
+    int t_n0;
+    double dt;
+    StepRef sr;
+};
+// A row's node, its first contribution and where the others stand.
+struct RowTerm {
+    float* f;
+    SrcTerm first;
+    int p, end;
+};
+// Source rows ride in the half step while they are few, at most one on 25 cells:
+// a launch less (84^3 with a box inset 15, one on 43: 20.5 us a step alone,
+// against 24.5 with k_sources).  A z face of a TF/SF box puts two rows of five
+// dependent loads on each of a warp's 128 cells, so where the box fills a small
+// grid a thread a row is faster (93x41x67, one on 13: 20.7 riding, 19.0 not).
+constexpr int kRowsAtOnce = 4;
+constexpr long long kCellsARow = 25;
+// Observations of one side's fields after step sr, one thread a point probe, a
+// volume probe's node or a surface sample.
+struct QuadObs {
+    KProbes probes;
+    int first_n;
+    int nvol;
+    VolProbe vol[kQuadVol];
+    int nfar;
+    FarArgs far;
+    int ox, oy, oz;
+    StepRef sr;
+};
+
+__device__ __forceinline__ void observe(const KGrid& g, const QuadObs& o, int side, long long q) {
+    const int n = step_of(o.sr);
+    if (q < o.probes.n) {
+        if ((o.probes.comp[q] >= 3) == (side == 1)) probe_one(g, o.probes, n, o.first_n, (int)q);
+        return;
+    }
+    q -= o.probes.n;
+    for (int v = 0; v < o.nvol; ++v) {
+        const VolProbe& p = o.vol[v];
+        if ((p.magnetic != 0) != (side == 1)) continue;
+        const long long nodes = (long long)p.ni * p.nj * p.nk;
+        if (q < nodes) {
+            if (p.kind == 0) vol_probe_node<true>(g, p, n, o.ox, o.oy, o.oz, nodes, q);
+            else vol_probe_node<false>(g, p, n, o.ox, o.oy, o.oz, nodes, q);
+            return;
+        }
+        q -= nodes;
+    }
+    int m;
+    if (o.nfar && q < o.far.samples && far_step(o.far, n, m)) far_sample(g, o.far, m, side ? 2 : 1, o.ox, o.oy, o.oz, (int)q);
+}
+
 template <int SIDE>
+__global__ void __launch_bounds__(kQuadThreads) k_observe(const __grid_constant__ KGrid g, const __grid_constant__ QuadObs o) {
+    grid_wait();
+    observe(g, o, SIDE, blockIdx.x * (long long)kQuadThreads + threadIdx.x);
+}
+
+// One half step: blocks below `blocks` march quads (bx of them a chunk of
+// planes) and apply the source rows on their cells; with OBS the blocks from
+// there on observe the other field, which this half step leaves alone.  A step
+// is then two launches, where the sources and each kind of observation took one
+// each (84^3 with a plane wave and probes: 5 launches, 24.0 us a step alone).
+template <int SIDE, bool OBS>
 __global__ void __launch_bounds__(kQuadThreads, 8)
-    k_quad(const __grid_constant__ QuadView g, const __grid_constant__ QuadSide s, int chunk) {
+    k_quad(const __grid_constant__ QuadView g, const __grid_constant__ QuadSide s, const __grid_constant__ KGrid kg,
+           const __grid_constant__ QuadSrc src, const __grid_constant__ std::conditional_t<OBS, QuadObs, char> obs, int chunk, int bx,
+           int blocks) {
+    if constexpr (OBS) {
+        if ((int)blockIdx.x >= blocks) {
+            grid_wait();
+            observe(kg, obs, 1 - SIDE, (blockIdx.x - blocks) * (long long)kQuadThreads + threadIdx.x);
+            return;
+        }
+    }
     // everything before grid_wait is constant over the run: it overlaps the
     // kernel before
     __shared__ float2 tab[256];
     __shared__ QuadLine zl[kQuadChunk];
+    __shared__ RowTerm ahead[kQuadThreads];
     for (int m = threadIdx.x; m < s.nmed1; m += kQuadThreads) tab[m] = s.tab[m];
-    int p = blockIdx.x * kQuadThreads + threadIdx.x;
+    const int by = blockIdx.x / bx;
+    int p = (blockIdx.x - by * bx) * kQuadThreads + threadIdx.x;
+    const int k0 = by * chunk, k1 = min(k0 + chunk, s.nz), kb = s.z0 + k0, ke = s.z0 + k1 - 1;
+    for (int m = threadIdx.x; m <= ke - kb; m += kQuadThreads) zl[m] = s.z[kb + m];
+    // the warp's source rows: their first contributions are formed here
+    int r0 = 0, r1 = 0, n = 0;
+    bool pw_on = false;
+    const int lane = threadIdx.x & 31;
+    if (src.ptr && p - lane < s.threads) {
+        const int* sp = src.ptr + (p >> 5) * s.nz;
+        r0 = sp[k0];
+        r1 = sp[k1];
+        if (r0 < r1) {
+            n = step_of(src.sr);
+            pw_on = __shfl_sync(0xffffffffu, lane == 0 ? (int)pw_switch_up(src.s, n, src.tiempo, src.t_n0, src.dt, SIDE) : 0, 0) != 0;
+            if (src.s.pw_only && !pw_on) r1 = r0;
+        }
+    }
+    float t = 0.0f, G21 = 0.0f;
+    if (r0 < r1) {
+        const double tn = src.tiempo[n - src.t_n0];
+        t = SIDE ? (float)(tn + (double)0.5f * src.dt) : (float)tn;
+        G21 = SIDE ? kg.gm2[1] : kg.g2[1];
+    }
+    auto row_of = [&](int r) {
+        const QuadRow q = src.row[r];
+        return RowTerm{kg.F[q.comp] + q.node, source_term(src.s, q.e, t, G21, 7, pw_on), q.first + 1, q.first + q.count};
+    };
+    if (r0 + lane < r1) ahead[threadIdx.x] = row_of(r0 + lane);
     const bool inner = p < s.inner;
     if (!inner) p -= s.inner;
-    const int w = inner ? s.nq - s.xlo - s.xhi : s.xlo + s.xhi, r = p / w;
+    const int w = inner ? s.nq - s.xlo - s.xhi : s.xlo + s.xhi, r = w ? p / w : s.ny;
     const bool valid = r < s.ny;
-    int q = p - r * w;
+    int q = valid ? p - r * w : 0;
     q = inner ? q + s.xlo : q < s.xlo ? q : q + (s.nq - w);
     const int j = s.y0 + (valid ? r : s.ny - 1), i = 4 * q;
-    const int kb = s.z0 + blockIdx.y * chunk, ke = min(kb + chunk, s.z0 + s.nz) - 1;
-    for (int m = threadIdx.x; m <= ke - kb; m += kQuadThreads) zl[m] = s.z[kb + m];
     const QuadX* X = s.x + (i >> 2);
     const QuadLine Y = ldl(s.y + j);
     float idx[4];
@@ -52,6 +166,36 @@ __global__ void __launch_bounds__(kQuadThreads, 8)
     grid_wait();
     if (__any_sync(0xffffffffu, meet != 0)) quad_march<SIDE, true>(g, s, tab, zl, X, Y, idx, meet, whole, i, j, kb, ke, valid);
     else quad_march<SIDE, false>(g, s, tab, zl, X, Y, idx, meet, whole, i, j, kb, ke, valid);
+    if (r0 < r1) {
+        __syncwarp();  // the warp's cells are stored
+        if (r0 + lane < r1) {
+            const RowTerm row = ahead[threadIdx.x];
+            float v = source_add(*row.f, row.first);
+            for (int e = row.p; e < row.end; ++e) v = source_add(v, source_term(src.s, src.s.e[e], t, G21, 7, pw_on));
+            *row.f = v;
+        }
+        for (int r = r0 + 32 + lane; r < r1; r += 32 * kRowsAtOnce) {
+            // on distinct nodes: the loads of several rows, then their stores
+            RowTerm row[kRowsAtOnce];
+            float v[kRowsAtOnce];
+#pragma unroll
+            for (int u = 0; u < kRowsAtOnce; ++u) {
+                row[u].f = nullptr;
+                if (r + 32 * u < r1) {
+                    row[u] = row_of(r + 32 * u);
+                    v[u] = *row[u].f;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kRowsAtOnce; ++u)
+                if (row[u].f) {
+                    v[u] = source_add(v[u], row[u].first);
+                    for (int e = row[u].p; e < row[u].end; ++e)
+                        v[u] = source_add(v[u], source_term(src.s, src.s.e[e], t, G21, 7, pw_on));
+                    *row[u].f = v[u];
+                }
+        }
+    }
 }
 
 __global__ void k_quad_tables(KGrid g, KCpml cp, int nxa, int nya, int nza, int side, QuadX* x, QuadLine* y, QuadLine* z,
@@ -106,7 +250,7 @@ namespace sgpu {
 
 bool quads_usable(const sgpu_ctx* c) { return tma_usable(c) && c->vol <= kQuadCells && !c->wait_drill; }
 
-QuadView quad_view(const sgpu_ctx* c) {
+static QuadView quad_view(const sgpu_ctx* c) {
     QuadView v{};
     const KGrid g = kgrid(c);
     for (int f = 0; f < 6; ++f) {
@@ -119,9 +263,8 @@ QuadView quad_view(const sgpu_ctx* c) {
     return v;
 }
 
-// The tables are built on first use and again after sgpu_init_cpml; before
-// steps are captured, so that a graph holds no allocation.
-sgpu_status quad_prepare(sgpu_ctx* c) {
+// The tables are built on first use and again after sgpu_init_cpml.
+static sgpu_status quad_prepare(sgpu_ctx* c) {
     if (c->quad_ok) return SGPU_OK;
     const size_t nx = c->pitch / 4, one = table_bytes(c);
     if (!c->quad_mem) {
@@ -141,7 +284,7 @@ sgpu_status quad_prepare(sgpu_ctx* c) {
     return SGPU_OK;
 }
 
-QuadSide quad_side(const sgpu_ctx* c, int side) {
+static QuadSide quad_side(const sgpu_ctx* c, int side) {
     const KGrid g = kgrid(c);
     const size_t nx = c->pitch / 4, one = table_bytes(c);
     QuadSide s{};
@@ -176,18 +319,134 @@ QuadSide quad_side(const sgpu_ctx* c, int side) {
     return s;
 }
 
-sgpu_status launch_quad(sgpu_ctx* c, int side) {
-    const sgpu_status st = quad_prepare(c);
+// The source rows grouped by (warp's quads, plane) of their node, in the
+// kernel's numbering of the quads.
+static sgpu_status quad_sources(sgpu_ctx* c) {
+    if (c->quad_src_ok) return SGPU_OK;
+    for (void* q : c->quad_src_allocs) ctx_free(c, q);
+    c->quad_src_allocs.clear();
+    c->quad_src_fits = true;
+    for (int side = 0; side < 2; ++side) {  // src_rows holds a side's rows where rows_ride
+        c->quad_sptr[side] = nullptr;
+        c->quad_srow[side] = nullptr;
+        const SrcRows& h = c->src_rows[side];
+        const size_t n = h.node.size();
+        if (n == 0 || !c->quad_src_fits) continue;
+        const QuadSide s = quad_side(c, side);
+        const int we = s.xlo + s.xhi, wi = s.nq - we;
+        const size_t keys = (size_t)((s.threads + 31) / 32) * s.nz;
+        std::vector<int> ptr(keys + 1, 0), key(n);
+        for (size_t r = 0; r < n; ++r) {
+            const int q = h.node[r] % c->pitch / 4, j = (int)(h.node[r] % c->plane) / c->pitch - s.y0,
+                      k = (int)(h.node[r] / c->plane) - s.z0;
+            if (h.comp[r] / 3 != side || q >= s.nq || j < 0 || j >= s.ny || k < 0 || k >= s.nz) {
+                c->quad_src_fits = false;  // no thread of the side updates this cell
+                break;
+            }
+            const bool in = q >= s.xlo && q < s.nq - s.xhi;
+            const int p = in ? j * wi + (q - s.xlo) : s.inner + j * we + (q < s.xlo ? q : q - wi);
+            key[r] = p / 32 * s.nz + k;
+            ++ptr[key[r] + 1];
+        }
+        if (!c->quad_src_fits) continue;
+        for (size_t q = 0; q < keys; ++q) ptr[q + 1] += ptr[q];
+        std::vector<int> at(ptr.begin(), ptr.end() - 1);
+        std::vector<QuadRow> row(n);
+        for (size_t r = 0; r < n; ++r)
+            row[at[key[r]]++] = QuadRow{h.node[r], h.comp[r], h.ptr[r + 1] - h.ptr[r], h.ptr[r], h.first[r]};
+        int* dp = (int*)ctx_malloc(c, ptr.size() * sizeof(int));
+        if (dp) c->quad_src_allocs.push_back(dp);
+        void* dr = ctx_malloc(c, n * sizeof(QuadRow));
+        if (dr) c->quad_src_allocs.push_back(dr);
+        if (!dp || !dr) return set_error(c, SGPU_ERR_OOM, "source rows by warp");
+        cudaError_t e = cudaMemcpyAsync(dp, ptr.data(), ptr.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(dr, row.data(), n * sizeof(QuadRow), cudaMemcpyHostToDevice, c->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+        if (e != cudaSuccess) return cuda_error(c, "source rows by warp", e);
+        c->quad_sptr[side] = dp;
+        c->quad_srow[side] = dr;
+    }
+    c->quad_src_ok = true;
+    return SGPU_OK;
+}
+
+bool rows_ride(const sgpu_ctx* c, int side) {
+    const QuadSide s = quad_side(c, side);
+    return kCellsARow * c->src[side].nrows <= 4ll * s.nq * s.ny * s.nz;
+}
+
+bool observers_ride(const sgpu_ctx* c) { return (int)c->vprobes.size() <= kQuadVol && c->farfields.size() <= 1; }
+
+// The observers of one side's fields and their threads (0: none).
+static QuadObs quad_obs(const sgpu_ctx* c, int side, StepRef sr, long long* threads) {
+    QuadObs o{};
+    o.probes = c->probes;
+    o.first_n = c->probe_first_n;
+    o.ox = c->ox; o.oy = c->oy; o.oz = c->oz;
+    o.sr = sr;
+    *threads = c->probes.n;
+    for (const VolProbe& v : c->vprobes) {
+        if ((v.magnetic != 0) != (side == 1)) continue;
+        o.vol[o.nvol++] = v;
+        *threads += (long long)v.ni * v.nj * v.nk;
+    }
+    for (const FarField& f : c->farfields)
+        if (f.samples) {
+            o.far = far_args(f);
+            o.nfar = 1;
+            *threads += f.samples;
+        }
+    return o;
+}
+
+sgpu_status launch_observe(sgpu_ctx* c, int side, StepRef sr) {
+    long long threads;
+    const QuadObs o = quad_obs(c, side, sr, &threads);
+    if (threads == 0) return SGPU_OK;
+    const unsigned blocks = (unsigned)((threads + kQuadThreads - 1) / kQuadThreads);
+    const cudaError_t e = side ? launch_after(c->stream, blocks, kQuadThreads, k_observe<1>, kgrid(c), o)
+                               : launch_after(c->stream, blocks, kQuadThreads, k_observe<0>, kgrid(c), o);
+    return e == cudaSuccess ? SGPU_OK : cuda_error(c, "k_observe", e);
+}
+
+sgpu_status launch_quad(sgpu_ctx* c, int side, StepRef sr, bool sources, const StepRef* obs, bool* applied) {
+    sgpu_status st = quad_prepare(c);
     if (st) return st;
     const QuadSide s = quad_side(c, side);
     const int bx = (s.threads + kQuadThreads - 1) / kQuadThreads;
     int chunk = kQuadChunk;
     while (chunk > 2 && (long long)bx * ((s.nz + chunk - 1) / chunk) < 148 * 16) chunk /= 2;
-    const dim3 grid(bx, (s.nz + chunk - 1) / chunk);
+    const int blocks = bx * ((s.nz + chunk - 1) / chunk);
     const QuadView v = quad_view(c);
-    const cudaError_t e = side ? launch_after(c->stream, grid, kQuadThreads, k_quad<1>, v, s, chunk)
-                               : launch_after(c->stream, grid, kQuadThreads, k_quad<0>, v, s, chunk);
+    const KGrid g = kgrid(c);
+    QuadSrc src{};
+    if (sources && rows_ride(c, side)) {
+        if ((st = quad_sources(c))) return st;
+        if (c->quad_src_fits) {
+            src = QuadSrc{c->quad_sptr[side], (const QuadRow*)c->quad_srow[side], c->src[side], c->d_tiempo, c->t_n0, c->dt, sr};
+            *applied = true;
+        }
+    }
+    cudaError_t e;
+    long long threads = 0;
+    QuadObs o{};
+    if (obs) o = quad_obs(c, 1 - side, *obs, &threads);
+    if (threads) {
+        const int all = blocks + (int)((threads + kQuadThreads - 1) / kQuadThreads);
+        e = side ? launch_after(c->stream, all, kQuadThreads, k_quad<1, true>, v, s, g, src, o, chunk, bx, blocks)
+                 : launch_after(c->stream, all, kQuadThreads, k_quad<0, true>, v, s, g, src, o, chunk, bx, blocks);
+    } else {
+        e = side ? launch_after(c->stream, blocks, kQuadThreads, k_quad<1, false>, v, s, g, src, '\0', chunk, bx, blocks)
+                 : launch_after(c->stream, blocks, kQuadThreads, k_quad<0, false>, v, s, g, src, '\0', chunk, bx, blocks);
+    }
     return e == cudaSuccess ? SGPU_OK : cuda_error(c, "k_quad", e);
+}
+
+// What steps need on the device before they are captured: a graph holds no
+// allocation.
+sgpu_status quad_ready(sgpu_ctx* c) {
+    const sgpu_status st = quad_prepare(c);
+    return st ? st : quad_sources(c);
 }
 
 }  // namespace sgpu

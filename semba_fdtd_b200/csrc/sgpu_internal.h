@@ -207,6 +207,13 @@ struct alignas(64) TMaps {
     CUtensorMap m[21];  // 9 field / media maps, then the 12 psi slabs of the side
 };
 
+// The source rows of a side on the host: node, component, where a row's
+// contributions start, and the first of them.
+struct SrcRows {
+    std::vector<int> node, comp, ptr;
+    std::vector<SrcEntry> first;
+};
+
 struct StepRef {
     const int* dev_n;  // if non-null, the step index is read from here
     int n;
@@ -304,6 +311,13 @@ struct sgpu_ctx {
     // tables of the quad kernels (quads.cu): one x table and two line tables a side
     void* quad_mem = nullptr;
     bool quad_ok = false;
+    // ... and the source rows by warp and plane (quad_src_fits: every row lies on
+    // a cell the kernels update)
+    sgpu::SrcRows src_rows[2];
+    int* quad_sptr[2] = {};
+    void* quad_srow[2] = {};
+    std::vector<void*> quad_src_allocs;
+    bool quad_src_ok = false, quad_src_fits = false;
     // scratch
     unsigned int* d_flag = nullptr;
     // TMA-pipelined fused kernels: tensor maps and the bounded-wait error word
@@ -365,8 +379,16 @@ void ctx_free(sgpu_ctx* c, void* p);
 // The curl + CPML half step of quads.cu (0 E, 1 H), its tables, and whether the
 // default kernel family takes it for this context.
 bool quads_usable(const sgpu_ctx* c);
-sgpu_status quad_prepare(sgpu_ctx* c);
-sgpu_status launch_quad(sgpu_ctx* c, int side);
+sgpu_status quad_ready(sgpu_ctx* c);
+// With `sources` the source rows of step sr are applied too when they can be
+// (*applied); with `obs` the observations of that step that read the other
+// field ride along (observers_ride).  launch_observe: those of one side alone.
+sgpu_status launch_quad(sgpu_ctx* c, int side, StepRef sr, bool sources, const StepRef* obs, bool* applied);
+bool rows_ride(const sgpu_ctx* c, int side);
+bool observers_ride(const sgpu_ctx* c);
+sgpu_status launch_observe(sgpu_ctx* c, int side, StepRef sr);
+struct FarArgs;
+FarArgs far_args(const FarField& F);
 // UpdateFarField for every far field of the context (farfield.cu).
 sgpu_status launch_farfields(sgpu_ctx* c, StepRef sr);
 void free_farfields(sgpu_ctx* c);

@@ -49,6 +49,50 @@ def test_ragged_quads_equal_the_oracle(n, layers, boundary):
             assert_bits_equal(s.field(c), o.field(c), err_msg=f"component {c}")
 
 
+@pytest.mark.parametrize("inset", [2, 5, 9])
+def test_rows_and_observers_in_the_half_steps(inset):
+    """A TF/SF box from one that fills the grid (source rows by k_sources) to a
+    small one (rows in the half step, several a lane on its z faces), with more
+    point probes than a block of observers, a volume probe of each kind and
+    field, and a step count that leaves a remainder after the captured steps."""
+    n = (41, 26, 23)
+    b = casegen._Builder(n, 75, 3)
+    b.steps([0.003], [0.003], [0.003])
+    ds = casegen.courant_dt(0.003) / 2
+    lo, hi = [inset] * 3, [v - inset for v in n]
+    b.planewave(lo, hi, 0.7, 1.9, 1.1, 0.4, "gauss.exc", ds, casegen.gaussian(ds, 20e-12, 60e-12, 0.2e-9))
+    b.nodal([v // 2 for v in n], [n[0] // 2, n[1] // 2, n[2] // 2 + 1], "dipole.exc", ds,
+            casegen.gaussian_derivative(ds, 8e-12, 40e-12, 0.1e-9))
+    rng = np.random.default_rng(inset)
+    for q in range(25):
+        pos = [int(rng.integers(1, v - 1)) for v in n]
+        b.probe(f"e{q}", "electric", pos, "xyz")
+        b.probe(f"h{q}", "magnetic", pos, "z")
+    pb = read_case(b.write(_DIR, f"rows_{inset}"))
+    box, freqs = (5, 20, 4, 15, 3, 12), (1e9, 3e9)
+    o = oracle.Oracle(pb)
+    ids = [o.add_freq_probe(m, box, (2, 1, 3), np.array(freqs, np.float32)) for m in (False, True)]
+    with Solver(pb) as s:
+        got = [s.add_freq_probe(m, box, (2, 1, 3), freqs) for m in (False, True)]
+        mov = [s.add_movie_probe(m, box, every=7, capacity=64) for m in (False, True)]
+        assert_bits_equal(s.run(), o.step(pb.nsteps + 1))
+        for c in range(6):
+            assert_bits_equal(s.field(c), o.field(c), err_msg=f"component {c}")
+        for a, r in zip(got, ids):
+            assert_bits_equal(s.freq_probe(a, 2), o.freq_probe(r))
+        for m, first in zip(mov, (0, 3)):
+            n0, frames = s.movie_frames(m)
+            assert n0 == 0 and len(frames) == 11
+            # the last frame is of step 70: compare with a fresh run to it
+            with Solver(pb, kernel_family=0) as w:
+                w.step(71)
+                for c in range(3):
+                    f = w.field(first + c)
+                    lo_ = [-a for a in (s.alloc[first + c][0], s.alloc[first + c][2], s.alloc[first + c][4])]
+                    want = f[5 + lo_[0]:21 + lo_[0], 4 + lo_[1]:16 + lo_[1], 3 + lo_[2]:13 + lo_[2]].transpose(2, 1, 0)
+                    assert_bits_equal(frames[-1][c], np.ascontiguousarray(want))
+
+
 @pytest.mark.parametrize("n", [(203, 187, 179), (301, 249, 197)])
 def test_both_sides_of_the_line_equal_the_oracle(n):
     """Just below and just above 16 Mi padded cells, where the quads hand over
