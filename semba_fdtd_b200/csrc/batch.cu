@@ -34,6 +34,7 @@
 // The persistent batched field kernels keep a 4-stage ring (3 CTAs an SM,
 // bound by their registers); the plain ones run 3 stages at 4 CTAs an SM.
 #define SGPU_TMA_STAGES 4
+#include "quads.cuh"
 #include "tma_fields.cuh"
 
 using namespace sgpu;
@@ -132,7 +133,7 @@ struct RangeItem {
     long long q0, q1;  // node / row / probe range
 };
 
-enum : int { kCntE = 0, kCntH, kCntNode, kCntSrcE, kCntSrcH, kCntProbe, kCntClone, kCntMur, kCntMNode, kNumCounts };
+enum : int { kCntE = 0, kCntH, kCntNode, kCntSrcE, kCntSrcH, kCntProbe, kCntClone, kCntMur, kCntMNode, kCntQuadE, kCntQuadH, kNumCounts };
 
 constexpr int kNodeChunk = 2048;  // ADE nodes per work item
 constexpr int kPhaseThreads = 256;
@@ -201,6 +202,59 @@ __global__ void __launch_bounds__(kBX * kBY, 4)
             if (w.cp) hfield_column<MODE, true>(g, V.cp, g.gm1, g.gm2, i, jc, w.kb, w.ke, vx, vy, vz);
             else hfield_column<MODE, false>(g, V.cp, g.gm1, g.gm2, i, jc, w.kb, w.ke, vx, vy, vz);
         }
+    }
+}
+
+// The half steps of small instances (quads.cuh): items are (slot, first of 64
+// quad threads in `ib`, planes kb..ke), taken in turn by resident blocks of two
+// warps.  A block holds the view of its instance in shared memory and the plane
+// lines of its item.
+struct QuadInst {
+    QuadView v;
+    QuadSide s[2];
+};
+static_assert(sizeof(QuadView) % 4 == 0 && sizeof(QuadSide) % 4 == 0, "copied by words");
+// Planes an item: 4, 8, 16, 32 took 956, 1004, 1074, 1265 us a step (24
+// instances, 42 M swept cells; the ring 1284); at 8 the host's lists are half
+// as long as at 4.
+constexpr int kBatchQuadThreads = 64, kBatchQuadChunk = 8, kBatchQuadBlocks = 8;
+template <int SIDE>
+__global__ void __launch_bounds__(kBatchQuadThreads, kBatchQuadBlocks)
+    k_batch_quad(const QuadInst* __restrict__ insts, const InstDesc* __restrict__ descs, const FieldItem* __restrict__ items,
+                 const int* counts, const int* G) {
+    __shared__ QuadView v;
+    __shared__ QuadSide s;
+    __shared__ float2 tab[256];
+    __shared__ QuadLine zl[kBatchQuadChunk];
+    const int n_items = counts[SIDE == 0 ? kCntQuadE : kCntQuadH];
+    int held = -1;
+    grid_wait();
+    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
+        const FieldItem w = items[it];
+        bool on;
+        inst_step(descs[w.slot], G, &on);
+        if (!on) continue;
+        __syncthreads();  // the block is done with the last item's lines and view
+        if (w.slot != held) {
+            held = w.slot;
+            const QuadInst& I = insts[w.slot];
+            for (int q = threadIdx.x; q < (int)(sizeof(QuadView) / 4); q += kBatchQuadThreads) ((int*)&v)[q] = ((const int*)&I.v)[q];
+            for (int q = threadIdx.x; q < (int)(sizeof(QuadSide) / 4); q += kBatchQuadThreads)
+                ((int*)&s)[q] = ((const int*)&I.s[SIDE])[q];
+            __syncthreads();
+            for (int m = threadIdx.x; m < s.nmed1; m += kBatchQuadThreads) tab[m] = s.tab[m];
+        }
+        for (int m = threadIdx.x; m <= w.ke - w.kb; m += kBatchQuadThreads) zl[m] = s.z[w.kb + m];
+        int i, j;
+        const bool valid = quad_at(s, w.ib + (int)threadIdx.x, i, j);
+        const QuadX* X = s.x + (i >> 2);
+        const QuadLine Y = ldl(s.y + j);
+        float idx[4];
+        ld4(idx, X->id);
+        const unsigned meet = valid ? X->meet & Y.hold : 0u, whole = X->whole;
+        __syncthreads();
+        if (__any_sync(0xffffffffu, meet != 0)) quad_march<SIDE, true>(v, s, tab, zl, X, Y, idx, meet, whole, i, j, w.kb, w.ke, valid);
+        else quad_march<SIDE, false>(v, s, tab, zl, X, Y, idx, meet, whole, i, j, w.kb, w.ke, valid);
     }
 }
 
@@ -334,6 +388,7 @@ __global__ void __launch_bounds__(kTmaThreads, 3)
 template <int NU, bool MAG>
 __global__ void __launch_bounds__(kPhaseThreads)
     k_batch_ade(const InstDesc* __restrict__ descs, const RangeItem* __restrict__ items, const int* counts, const int* G) {
+    grid_wait();
     const int n_items = counts[MAG ? kCntMNode : kCntNode];
     for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const RangeItem w = items[it];
@@ -362,6 +417,7 @@ __global__ void __launch_bounds__(kPhaseThreads)
 __global__ void __launch_bounds__(kPhaseThreads)
     k_batch_sources(const InstDesc* __restrict__ descs, const RangeItem* __restrict__ items, const int* counts, const int* G,
                     int side) {
+    grid_wait();
     const int n_items = counts[side == 0 ? kCntSrcE : kCntSrcH];
     for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const RangeItem w = items[it];
@@ -382,6 +438,7 @@ __global__ void __launch_bounds__(kPhaseThreads)
 // the device).
 __global__ void __launch_bounds__(kPhaseThreads)
     k_batch_probes(const InstDesc* __restrict__ descs, const RangeItem* __restrict__ items, const int* counts, const int* G) {
+    grid_wait();
     const int n_items = counts[kCntProbe];
     for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const RangeItem w = items[it];
@@ -399,6 +456,7 @@ __global__ void __launch_bounds__(kPhaseThreads)
 __global__ void __launch_bounds__(kPhaseThreads)
     k_batch_borders(const InstDesc* __restrict__ descs, const RangeItem* __restrict__ items, const int* counts, const int* G,
                     int which) {
+    grid_wait();
     const int n_items = counts[which == 0 ? kCntClone : kCntMur];
     for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const RangeItem w = items[it];
@@ -414,13 +472,17 @@ __global__ void __launch_bounds__(kPhaseThreads)
 }
 
 // The batch counter moves on by one step.
-__global__ void k_batch_tick(int* G) { *G += 1; }
+__global__ void k_batch_tick(int* G) {
+    grid_wait();
+    *G += 1;
+}
 
 struct Slot {
     sgpu_ctx* ctx = nullptr;
     int start = 0;   // batch counter value at the instance's step 0
     int nsteps = 0;  // last step index advanced (steps 0..nsteps)
     int size_class = 0;
+    bool quads = false;  // small enough for the quad kernels, and its tables are built
     bool reserved = false;  // an instance is being set up for this slot
 };
 
@@ -459,6 +521,11 @@ struct sgpu_batch {
     int* d_counts = nullptr;
     int* d_G = nullptr;
     FieldItem* d_field[2] = {};
+    // instances the quad kernels serve: their views by slot, and their items
+    QuadInst* d_quad_inst = nullptr;
+    FieldItem* d_quad[2] = {};
+    size_t cap_quad[2] = {};
+    bool any_quad = false, any_ring = false;  // of the listed instances
     RangeItem* d_node = nullptr;
     RangeItem* d_mnode = nullptr;  // magnetic ADE node ranges
     size_t cap_mnode = 0;
@@ -479,6 +546,8 @@ struct sgpu_batch {
     int ctas_per_sm = 4;
     // graph of kGraphSteps steps
     cudaGraphExec_t graph = nullptr;
+    bool graph_quad = false, graph_ring = false;
+    bool quads_ok = true;  // the quad kernels serve the batch (its lists were built for that)
     int graph_nu = 0, graph_ctas = 0;
     bool graph_tma = false, graph_border[2] = {}, graph_mnode = false;
     long long graph_wait = -1;
@@ -557,9 +626,10 @@ bool running(const Slot& s, int G) { return s.ctx && G - s.start <= s.nsteps; }
 
 // Rebuild the flattened work lists from the instances that still run.
 sgpu_status rebuild(sgpu_batch* b) {
-    std::vector<FieldItem> fi[2];
+    std::vector<FieldItem> fi[2], qi[2];
     std::vector<RangeItem> node, mnode, src[2], probe, border[2];
     int nu = 1;
+    b->quads_ok = b->family == 1 && !b->wait_drill;
     b->listed.assign(b->slots.size(), 0);
     for (int sl = 0; sl < (int)b->slots.size(); ++sl) {
         const Slot& s = b->slots[sl];
@@ -567,7 +637,14 @@ sgpu_status rebuild(sgpu_batch* b) {
         b->listed[sl] = 1;
         sgpu_ctx* c = s.ctx;
         const int chunk = b->chunk[s.size_class];
-        for (int side = 0; side < 2; ++side) {
+        const bool quads = b->quads_ok && b->slots[sl].quads;
+        for (int side = 0; side < 2 && quads; ++side) {
+            const QuadSide q = quad_side(c, side);
+            for (int kb = q.z0; kb < q.z0 + q.nz; kb += kBatchQuadChunk)
+                for (int p = 0; p < q.threads; p += kBatchQuadThreads)
+                    qi[side].push_back(FieldItem{sl, p, 0, kb, std::min(kb + kBatchQuadChunk, q.z0 + q.nz) - 1, 0});
+        }
+        for (int side = 0; side < 2 && !quads; ++side) {
             const int c0 = side ? 3 : 0;
             int x1 = -1, y0 = 1 << 30, y1 = -1, z0 = 1 << 30, z1 = -1;
             for (int f = c0; f < c0 + 3; ++f) {
@@ -610,6 +687,8 @@ sgpu_status rebuild(sgpu_batch* b) {
     sgpu_status s;
     for (int side = 0; side < 2; ++side) {
         if ((s = ensure(b, &b->d_field[side], &b->cap_field[side], fi[side].size()))) return s;
+        if ((s = ensure(b, &b->d_quad[side], &b->cap_quad[side], qi[side].size()))) return s;
+        if ((s = upload(b, b->d_quad[side], qi[side]))) return s;
         if ((s = ensure(b, &b->d_src[side], &b->cap_src[side], src[side].size()))) return s;
     }
     if ((s = ensure(b, &b->d_node, &b->cap_node, node.size())) || (s = ensure(b, &b->d_probe, &b->cap_probe, probe.size())))
@@ -625,6 +704,10 @@ sgpu_status rebuild(sgpu_batch* b) {
         (s = upload(b, b->d_src[0], src[0])) || (s = upload(b, b->d_src[1], src[1])) || (s = upload(b, b->d_probe, probe)))
         return s;
     std::vector<int> counts(kNumCounts);
+    b->any_quad = !qi[0].empty();
+    b->any_ring = !fi[0].empty();
+    counts[kCntQuadE] = (int)qi[0].size();
+    counts[kCntQuadH] = (int)qi[1].size();
     counts[kCntE] = (int)fi[0].size();
     counts[kCntH] = (int)fi[1].size();
     counts[kCntNode] = (int)node.size();
@@ -666,7 +749,7 @@ bool use_tma(const sgpu_batch* b) {
 }
 
 template <int NU, bool MAG> void ade_batch(sgpu_batch* b, int grid) {
-    k_batch_ade<NU, MAG><<<grid, kPhaseThreads, 0, b->stream>>>(b->d_desc, MAG ? b->d_mnode : b->d_node, b->d_counts, b->d_G);
+    launch_after(b->stream, grid, kPhaseThreads, k_batch_ade<NU, MAG>, b->d_desc, MAG ? b->d_mnode : b->d_node, b->d_counts, b->d_G);
 }
 
 template <bool MAG> void ade_phase(sgpu_batch* b, int grid) {
@@ -690,34 +773,41 @@ sgpu_status enqueue_step(sgpu_batch* b, cudaEvent_t* marks = nullptr) {
     auto mark = [&](int q) {
         if (marks) cudaEventRecord(marks[q], b->stream);
     };
-    if (tma) {
+    const int qgrid = b->num_sms * kBatchQuadBlocks;
+    if (b->any_quad)
+        launch_after(b->stream, qgrid, kBatchQuadThreads, k_batch_quad<0>, b->d_quad_inst, b->d_desc, b->d_quad[0], b->d_counts,
+                     b->d_G);
+    if (tma && b->any_ring) {
         cudaMemsetAsync(b->d_next, 0, 2 * sizeof(int), b->stream);  // the launches' item counters
         k_batch_tma_field<0><<<tgrid, kTmaThreads, kTmaSmem, b->stream>>>(b->d_desc, b->d_maps, b->d_field[0], b->d_counts,
                                                                           b->d_G, b->d_err, b->wait_cycles, b->wait_drill,
                                                                           b->d_next);
-    }
-    else
+    } else if (b->any_ring) {
         k_batch_field<0><<<grid, blk, 0, b->stream>>>(b->d_desc, b->d_field[0], b->d_counts, b->d_G);
+    }
     mark(0);
     ade_phase<false>(b, grid);
     mark(1);
-    k_batch_sources<<<grid, kPhaseThreads, 0, b->stream>>>(b->d_desc, b->d_src[0], b->d_counts, b->d_G, 0);
+    launch_after(b->stream, grid, kPhaseThreads, k_batch_sources, b->d_desc, b->d_src[0], b->d_counts, b->d_G, 0);
     mark(2);
-    if (tma)
+    if (b->any_quad)
+        launch_after(b->stream, qgrid, kBatchQuadThreads, k_batch_quad<1>, b->d_quad_inst, b->d_desc, b->d_quad[1], b->d_counts,
+                     b->d_G);
+    if (tma && b->any_ring)
         k_batch_tma_field<1><<<tgrid, kTmaThreads, kTmaSmem, b->stream>>>(b->d_desc, b->d_maps, b->d_field[1], b->d_counts,
                                                                           b->d_G, b->d_err, b->wait_cycles, b->wait_drill,
                                                                           b->d_next + 1);
-    else
+    else if (b->any_ring)
         k_batch_field<1><<<grid, blk, 0, b->stream>>>(b->d_desc, b->d_field[1], b->d_counts, b->d_G);
     mark(3);
     if (b->any_mnode) ade_phase<true>(b, grid);
-    k_batch_sources<<<grid, kPhaseThreads, 0, b->stream>>>(b->d_desc, b->d_src[1], b->d_counts, b->d_G, 1);
+    launch_after(b->stream, grid, kPhaseThreads, k_batch_sources, b->d_desc, b->d_src[1], b->d_counts, b->d_G, 1);
     for (int w = 0; w < 2; ++w)
         if (b->any_border[w])
-            k_batch_borders<<<grid, kPhaseThreads, 0, b->stream>>>(b->d_desc, b->d_border[w], b->d_counts, b->d_G, w);
+            launch_after(b->stream, grid, kPhaseThreads, k_batch_borders, b->d_desc, b->d_border[w], b->d_counts, b->d_G, w);
     mark(4);
-    k_batch_probes<<<grid, kPhaseThreads, 0, b->stream>>>(b->d_desc, b->d_probe, b->d_counts, b->d_G);
-    k_batch_tick<<<1, 1, 0, b->stream>>>(b->d_G);
+    launch_after(b->stream, grid, kPhaseThreads, k_batch_probes, b->d_desc, b->d_probe, b->d_counts, b->d_G);
+    launch_after(b->stream, 1, 1, k_batch_tick, b->d_G);
     mark(5);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return berr(b, SGPU_ERR_CUDA, std::string("batched step launch: ") + cudaGetErrorString(e));
@@ -727,7 +817,7 @@ sgpu_status enqueue_step(sgpu_batch* b, cudaEvent_t* marks = nullptr) {
 sgpu_status ensure_graph(sgpu_batch* b) {
     if (b->graph && b->graph_nu == b->nu_max && b->graph_ctas == b->ctas_per_sm && b->graph_tma == use_tma(b) &&
         b->graph_border[0] == b->any_border[0] && b->graph_border[1] == b->any_border[1] &&
-        b->graph_mnode == b->any_mnode && b->graph_wait == b->wait_cycles && b->graph_drill == b->wait_drill)
+        b->graph_mnode == b->any_mnode && b->graph_quad == b->any_quad && b->graph_ring == b->any_ring && b->graph_wait == b->wait_cycles && b->graph_drill == b->wait_drill)
         return SGPU_OK;
     if (b->graph) {
         cudaGraphExecDestroy(b->graph);
@@ -755,6 +845,8 @@ sgpu_status ensure_graph(sgpu_batch* b) {
     b->graph_border[0] = b->any_border[0];
     b->graph_border[1] = b->any_border[1];
     b->graph_mnode = b->any_mnode;
+    b->graph_quad = b->any_quad;
+    b->graph_ring = b->any_ring;
     b->graph_wait = b->wait_cycles;
     b->graph_drill = b->wait_drill;
     return SGPU_OK;
@@ -827,6 +919,7 @@ sgpu_status sgpu_batch_create(uint64_t arena_bytes, int max_instances, sgpu_batc
     b->has_maps.assign(max_instances, 0);
     BTRY(b, cudaMalloc((void**)&b->d_desc, sizeof(InstDesc) * max_instances));
     BTRY(b, cudaMalloc((void**)&b->d_maps, sizeof(TMaps) * 2 * max_instances));
+    BTRY(b, cudaMalloc((void**)&b->d_quad_inst, sizeof(QuadInst) * max_instances));
     BTRY(b, cudaMalloc((void**)&b->d_err, sizeof(int)));
     BTRY(b, cudaMalloc((void**)&b->d_next, 2 * sizeof(int)));
     BTRY(b, cudaMalloc((void**)&b->d_counts, sizeof(int) * kNumCounts));
@@ -854,12 +947,14 @@ void sgpu_batch_destroy(sgpu_batch* b) {
     if (b->graph) cudaGraphExecDestroy(b->graph);
     cudaFree(b->d_desc);
     cudaFree(b->d_maps);
+    cudaFree(b->d_quad_inst);
     cudaFree(b->d_err);
     cudaFree(b->d_next);
     cudaFree(b->d_counts);
     cudaFree(b->d_G);
     for (int s = 0; s < 2; ++s) {
         cudaFree(b->d_field[s]);
+        cudaFree(b->d_quad[s]);
         cudaFree(b->d_src[s]);
     }
     cudaFree(b->d_node);
@@ -917,6 +1012,7 @@ sgpu_status sgpu_batch_add(sgpu_batch* b, const sgpu_problem* p, sgpu_ctx* plan,
     }
     if (!s) s = host_create_in(p, plan, nsteps, &b->arena, st, &c);
     if (!s) s = rebuild_sources(c);
+    const bool quads = !s && quads_usable(c) && quad_prepare(c) == SGPU_OK;
     if (!s && cudaEventRecord(ev, st) != cudaSuccess) {
         cudaGetLastError();
         s = SGPU_ERR_CUDA;
@@ -947,6 +1043,11 @@ sgpu_status sgpu_batch_add(sgpu_batch* b, const sgpu_problem* p, sgpu_ctx* plan,
     S.start = b->G;
     S.nsteps = nsteps;
     S.size_class = size_class_of(c);
+    S.quads = quads;
+    if (quads) {
+        const QuadInst I{quad_view(c), {quad_side(c, 0), quad_side(c, 1)}};
+        BTRY(b, cudaMemcpyAsync(b->d_quad_inst + sl, &I, sizeof(I), cudaMemcpyHostToDevice, b->stream));
+    }
     InstDesc D = make_desc(S, true);
     BTRY(b, cudaMemcpyAsync(b->d_desc + sl, &D, sizeof(InstDesc), cudaMemcpyHostToDevice, b->stream));
     b->has_maps[sl] = tma_usable(c) ? 1 : 0;
@@ -1001,6 +1102,7 @@ sgpu_status sgpu_batch_set_wait_drill(sgpu_batch* b, int on) {
     std::lock_guard<std::mutex> lock(b->mu);
     if (!b) return SGPU_ERR_ARG;
     b->wait_drill = on ? 1 : 0;
+    b->dirty = true;  // the drill is the ring's
     return SGPU_OK;
 }
 
@@ -1009,6 +1111,7 @@ sgpu_status sgpu_batch_set_kernel_family(sgpu_batch* b, int family) {
     std::lock_guard<std::mutex> lock(b->mu);
     if (!b || family < 0 || family > 1) return SGPU_ERR_ARG;
     b->family = family;
+    b->dirty = true;  // each family has its own lists
     return SGPU_OK;
 }
 

@@ -888,7 +888,8 @@ void sgpu_destroy(sgpu_ctx* c) {
     free_list(c, c->probe_allocs);
     free_list(c, c->vprobe_allocs);
     free_farfields(c);
-    dev_free(c, c->quad_mem);
+    if (c->quad_mem && c->arena) cudaFreeAsync(c->quad_mem, c->stream);
+    else dev_free(c, c->quad_mem);
     free_list(c, c->quad_src_allocs);
     if (c->stream && c->own_stream) cudaStreamDestroy(c->stream);
     if (c->host && c->host_free) c->host_free(c->host);

@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kQuadThreads, 8)
     __shared__ RowTerm ahead[kQuadThreads];
     for (int m = threadIdx.x; m < s.nmed1; m += kQuadThreads) tab[m] = s.tab[m];
     const int by = blockIdx.x / bx;
-    int p = (blockIdx.x - by * bx) * kQuadThreads + threadIdx.x;
+    const int p = (blockIdx.x - by * bx) * kQuadThreads + threadIdx.x;
     const int k0 = by * chunk, k1 = min(k0 + chunk, s.nz), kb = s.z0 + k0, ke = s.z0 + k1 - 1;
     for (int m = threadIdx.x; m <= ke - kb; m += kQuadThreads) zl[m] = s.z[kb + m];
     // the warp's source rows: their first contributions are formed here
@@ -150,13 +150,8 @@ __global__ void __launch_bounds__(kQuadThreads, 8)
         return RowTerm{kg.F[q.comp] + q.node, source_term(src.s, q.e, t, G21, 7, pw_on), q.first + 1, q.first + q.count};
     };
     if (r0 + lane < r1) ahead[threadIdx.x] = row_of(r0 + lane);
-    const bool inner = p < s.inner;
-    if (!inner) p -= s.inner;
-    const int w = inner ? s.nq - s.xlo - s.xhi : s.xlo + s.xhi, r = w ? p / w : s.ny;
-    const bool valid = r < s.ny;
-    int q = valid ? p - r * w : 0;
-    q = inner ? q + s.xlo : q < s.xlo ? q : q + (s.nq - w);
-    const int j = s.y0 + (valid ? r : s.ny - 1), i = 4 * q;
+    int i, j;
+    const bool valid = quad_at(s, p, i, j);
     const QuadX* X = s.x + (i >> 2);
     const QuadLine Y = ldl(s.y + j);
     float idx[4];
@@ -250,7 +245,7 @@ namespace sgpu {
 
 bool quads_usable(const sgpu_ctx* c) { return tma_usable(c) && c->vol <= kQuadCells && !c->wait_drill; }
 
-static QuadView quad_view(const sgpu_ctx* c) {
+QuadView quad_view(const sgpu_ctx* c) {
     QuadView v{};
     const KGrid g = kgrid(c);
     for (int f = 0; f < 6; ++f) {
@@ -264,11 +259,20 @@ static QuadView quad_view(const sgpu_ctx* c) {
 }
 
 // The tables are built on first use and again after sgpu_init_cpml.
-static sgpu_status quad_prepare(sgpu_ctx* c) {
+sgpu_status quad_prepare(sgpu_ctx* c) {
     if (c->quad_ok) return SGPU_OK;
     const size_t nx = c->pitch / 4, one = table_bytes(c);
     if (!c->quad_mem) {
-        c->quad_mem = ctx_malloc(c, 2 * one);
+        // in a batch, too, from the device's pool: the arena holds what an
+        // instance's footprint counts
+        if (c->arena) {
+            if (cudaMallocAsync(&c->quad_mem, 2 * one, c->stream) != cudaSuccess) {
+                cudaGetLastError();
+                c->quad_mem = nullptr;
+            }
+        } else {
+            c->quad_mem = ctx_malloc(c, 2 * one);
+        }
         if (!c->quad_mem) return set_error(c, SGPU_ERR_OOM, "quad tables");
     }
     for (int h = 0; h < 2; ++h) {
@@ -284,7 +288,7 @@ static sgpu_status quad_prepare(sgpu_ctx* c) {
     return SGPU_OK;
 }
 
-static QuadSide quad_side(const sgpu_ctx* c, int side) {
+QuadSide quad_side(const sgpu_ctx* c, int side) {
     const KGrid g = kgrid(c);
     const size_t nx = c->pitch / 4, one = table_bytes(c);
     QuadSide s{};

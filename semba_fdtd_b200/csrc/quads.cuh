@@ -48,7 +48,26 @@ struct QuadView {
     int sw[6][6];
 };
 
+// Views of a context, and its tables (built on first use).
+QuadView quad_view(const sgpu_ctx* c);
+QuadSide quad_side(const sgpu_ctx* c, int side);
+sgpu_status quad_prepare(sgpu_ctx* c);
+
 namespace dev {
+
+// The quad of thread p of a side: its first cell and row; false past the last
+// (which then names a valid quad all the same).
+__device__ __forceinline__ bool quad_at(const QuadSide& s, int p, int& i, int& j) {
+    const bool inner = p < s.inner;
+    if (!inner) p -= s.inner;
+    const int w = inner ? s.nq - s.xlo - s.xhi : s.xlo + s.xhi, r = w ? p / w : s.ny;
+    const bool valid = r < s.ny;
+    int q = valid ? p - r * w : 0;
+    q = inner ? q + s.xlo : q < s.xlo ? q : q + (s.nq - w);
+    j = s.y0 + (valid ? r : s.ny - 1);
+    i = 4 * q;
+    return valid;
+}
 
 __device__ __forceinline__ void ld4(float (&v)[4], const float* p) {
     const float4 q = *(const float4*)p;

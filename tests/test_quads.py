@@ -105,3 +105,25 @@ def test_both_sides_of_the_line_equal_the_oracle(n):
         for c in range(6):
             assert_bits_equal(s.field(c), o.field(c), err_msg=f"component {c}")
 
+
+
+def test_batch_of_small_and_large_instances():
+    """Quads and TMA ring in one batch: an instance above the line next to one
+    below it, a join while the large one runs, and a switch of families."""
+    from semba_fdtd_b200.batch import Batch
+    big, _ = _case((301, 249, 197), 6)
+    small, _ = _case((27, 7, 5), 1)
+    wide, _ = _case((61, 40, 37), 5)
+    pbs = [replace(big, nsteps=5), replace(small, nsteps=9), replace(wide, nsteps=7)]
+    want = [oracle.Oracle(pb).step(pb.nsteps + 1) for pb in pbs]
+    with Batch(4 << 30, 4) as b:
+        slots = [b.add(pbs[0]), b.add(pbs[1])]
+        b.advance(2)
+        slots.append(b.add(pbs[2]))
+        b.advance(2)
+        b._check(b.lib.sgpu_batch_set_kernel_family(b._h, 0), "family")
+        b.advance(1)
+        b._check(b.lib.sgpu_batch_set_kernel_family(b._h, 1), "family")
+        b.run_all()
+        for s, w in zip(slots, want):
+            assert_bits_equal(b.probes(s), w)
