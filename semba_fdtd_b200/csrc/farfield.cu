@@ -542,12 +542,12 @@ sgpu_status sgpu_farfield_transform(sgpu_ctx* c, int id, const sgpu_farfield_ang
     double2* d_dft = nullptr;
     double* d_rows = nullptr;
     const int nc = (int)cells.size(), nd = (int)dirs.size();
-    cudaError_t e = cudaMalloc(&d_cells, sizeof(TCell) * nc);
-    if (e == cudaSuccess) e = cudaMalloc(&d_cur, sizeof(Currents) * (size_t)nc * F.nf);
-    if (e == cudaSuccess) e = cudaMalloc(&d_dirs, sizeof(Dir) * nd);
-    if (e == cudaSuccess) e = cudaMalloc(&d_freq, sizeof(float) * F.nf);
-    if (e == cudaSuccess) e = cudaMalloc(&d_dft, sizeof(double2) * F.nf);
-    if (e == cudaSuccess) e = cudaMalloc(&d_rows, sizeof(double) * 9 * (size_t)need);
+    cudaError_t e = cudaMallocAsync(&d_cells, sizeof(TCell) * nc, c->stream);
+    if (e == cudaSuccess) e = cudaMallocAsync(&d_cur, sizeof(Currents) * (size_t)nc * F.nf, c->stream);
+    if (e == cudaSuccess) e = cudaMallocAsync(&d_dirs, sizeof(Dir) * nd, c->stream);
+    if (e == cudaSuccess) e = cudaMallocAsync(&d_freq, sizeof(float) * F.nf, c->stream);
+    if (e == cudaSuccess) e = cudaMallocAsync(&d_dft, sizeof(double2) * F.nf, c->stream);
+    if (e == cudaSuccess) e = cudaMallocAsync(&d_rows, sizeof(double) * 9 * (size_t)need, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_cells, cells.data(), sizeof(TCell) * nc, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_dirs, dirs.data(), sizeof(Dir) * nd, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_freq, F.freq.data(), sizeof(float) * F.nf, cudaMemcpyHostToDevice, c->stream);
@@ -564,12 +564,12 @@ sgpu_status sgpu_farfield_transform(sgpu_ctx* c, int id, const sgpu_farfield_ang
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, d_rows, sizeof(double) * 9 * (size_t)need, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    cudaFree(d_cells);
-    cudaFree(d_cur);
-    cudaFree(d_dirs);
-    cudaFree(d_freq);
-    cudaFree(d_dft);
-    cudaFree(d_rows);
+    if (d_cells) cudaFreeAsync(d_cells, c->stream);
+    if (d_cur) cudaFreeAsync(d_cur, c->stream);
+    if (d_dirs) cudaFreeAsync(d_dirs, c->stream);
+    if (d_freq) cudaFreeAsync(d_freq, c->stream);
+    if (d_dft) cudaFreeAsync(d_dft, c->stream);
+    if (d_rows) cudaFreeAsync(d_rows, c->stream);
     if (e != cudaSuccess) return set_error(c, SGPU_ERR_CUDA, std::string("far-field transform: ") + cudaGetErrorString(e));
     return SGPU_OK;
 }

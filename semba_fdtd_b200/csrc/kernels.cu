@@ -844,6 +844,7 @@ sgpu_status sgpu::create_in(const sgpu_grid_desc* d, Arena* arena, cudaStream_t 
     if ((s = dalloc(c, &c->d_flag, 1))) return fail(s);
     if ((s = dalloc(c, &c->d_err, 1))) return fail(s);
     CUDA_TRY(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
+    if ((s = quad_alloc(c))) return fail(s);
     c->tma_ready = build_tensor_maps(c);
     if (c->tma_ready) {
         const int smax = (int)(kTmaSmem + 2 * kShTable * sizeof(float));
@@ -1708,10 +1709,12 @@ sgpu_status sgpu_read_probes(sgpu_ctx* c, float* out, int max_steps, int* nsteps
     if (take <= 0) return SGPU_OK;
     if (!out) return set_error(c, SGPU_ERR_ARG, "null output");
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    // the rows are contiguous up to the ring's end: one copy, or two
     const int np = c->probes.n, cap = c->probes.cap;
-    for (long long r = 0; r < take; ++r) {
-        long long row = (c->probe_read + r) % cap;
-        CUDA_TRY(c, cudaMemcpy(out + r * np, c->probes.ring + row * np, np * sizeof(float), cudaMemcpyDeviceToHost));
+    for (long long r = 0; r < take;) {
+        const long long row = (c->probe_read + r) % cap, run = std::min<long long>(take - r, cap - row);
+        CUDA_TRY(c, cudaMemcpy(out + r * np, c->probes.ring + row * np, run * np * sizeof(float), cudaMemcpyDeviceToHost));
+        r += run;
     }
     c->probe_read += take;
     *nsteps = (int)take;
@@ -1865,9 +1868,10 @@ sgpu_status sgpu_read_movie_probe(sgpu_ctx* c, int id, float* out, int max_frame
     if (!out) return set_error(c, SGPU_ERR_ARG, "null output");
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     const size_t frame = (size_t)p.ni * p.nj * p.nk * 3;
-    for (long long r = 0; r < take; ++r) {
-        const long long slot = (read + r) % p.cap;
-        CUDA_TRY(c, cudaMemcpy(out + r * frame, p.ring + slot * frame, frame * sizeof(float), cudaMemcpyDeviceToHost));
+    for (long long r = 0; r < take;) {  // contiguous up to the ring's end
+        const long long slot = (read + r) % p.cap, run = std::min<long long>(take - r, p.cap - slot);
+        CUDA_TRY(c, cudaMemcpy(out + r * frame, p.ring + slot * frame, run * frame * sizeof(float), cudaMemcpyDeviceToHost));
+        r += run;
     }
     read += take;
     *frames = (int)take;

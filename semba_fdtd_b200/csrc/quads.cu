@@ -243,7 +243,7 @@ size_t table_bytes(const sgpu_ctx* c) {
 
 namespace sgpu {
 
-bool quads_usable(const sgpu_ctx* c) { return tma_usable(c) && c->vol <= kQuadCells && !c->wait_drill; }
+bool quads_usable(const sgpu_ctx* c) { return tma_usable(c) && c->vol <= kQuadCells && !c->wait_drill && c->quad_mem; }
 
 QuadView quad_view(const sgpu_ctx* c) {
     QuadView v{};
@@ -258,23 +258,25 @@ QuadView quad_view(const sgpu_ctx* c) {
     return v;
 }
 
+// Room for the tables, taken with the context's other buffers, so that a
+// context set up after another finds the pool's free blocks whole.  In a batch,
+// too, from the device's pool: the arena holds what an instance's footprint
+// counts.
+sgpu_status quad_alloc(sgpu_ctx* c) {
+    if (c->vol > kQuadCells) return SGPU_OK;
+    const size_t bytes = 2 * table_bytes(c);
+    if (!c->arena) c->quad_mem = ctx_malloc(c, bytes);
+    else if (cudaMallocAsync(&c->quad_mem, bytes, c->stream) != cudaSuccess) {
+        cudaGetLastError();
+        c->quad_mem = nullptr;
+    }
+    return c->quad_mem ? SGPU_OK : set_error(c, SGPU_ERR_OOM, "quad tables");
+}
+
 // The tables are built on first use and again after sgpu_init_cpml.
 sgpu_status quad_prepare(sgpu_ctx* c) {
     if (c->quad_ok) return SGPU_OK;
     const size_t nx = c->pitch / 4, one = table_bytes(c);
-    if (!c->quad_mem) {
-        // in a batch, too, from the device's pool: the arena holds what an
-        // instance's footprint counts
-        if (c->arena) {
-            if (cudaMallocAsync(&c->quad_mem, 2 * one, c->stream) != cudaSuccess) {
-                cudaGetLastError();
-                c->quad_mem = nullptr;
-            }
-        } else {
-            c->quad_mem = ctx_malloc(c, 2 * one);
-        }
-        if (!c->quad_mem) return set_error(c, SGPU_ERR_OOM, "quad tables");
-    }
     for (int h = 0; h < 2; ++h) {
         QuadX* x = (QuadX*)((char*)c->quad_mem + h * one);
         QuadLine* y = (QuadLine*)(x + nx);

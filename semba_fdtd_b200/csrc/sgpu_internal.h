@@ -379,6 +379,7 @@ void ctx_free(sgpu_ctx* c, void* p);
 // The curl + CPML half step of quads.cu (0 E, 1 H), its tables, and whether the
 // default kernel family takes it for this context.
 bool quads_usable(const sgpu_ctx* c);
+sgpu_status quad_alloc(sgpu_ctx* c);
 sgpu_status quad_ready(sgpu_ctx* c);
 // With `sources` the source rows of step sr are applied too when they can be
 // (*applied); with `obs` the observations of that step that read the other
