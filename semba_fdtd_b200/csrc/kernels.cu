@@ -1937,12 +1937,22 @@ sgpu_status note_probe_rows(sgpu_ctx* c, int n0, int count) {
         if (!ready(c)) return set_error((c), SGPU_ERR_STATE, "media matrices not uploaded");      \
     } while (0)
 
-sgpu_status sgpu_advance_ex(sgpu_ctx* c) { SGPU_READY(c); return launch_e<kBulk | kCx>(c); }
-sgpu_status sgpu_advance_ey(sgpu_ctx* c) { SGPU_READY(c); return launch_e<kBulk | kCy>(c); }
-sgpu_status sgpu_advance_ez(sgpu_ctx* c) { SGPU_READY(c); return launch_e<kBulk | kCz>(c); }
+sgpu_status sgpu_advance_ex(sgpu_ctx* c) {
+    SGPU_READY(c);
+    return c->family == 1 && quads_usable(c) ? launch_quad_part(c, 0, 0) : launch_e<kBulk | kCx>(c);
+}
+sgpu_status sgpu_advance_ey(sgpu_ctx* c) {
+    SGPU_READY(c);
+    return c->family == 1 && quads_usable(c) ? launch_quad_part(c, 0, 1) : launch_e<kBulk | kCy>(c);
+}
+sgpu_status sgpu_advance_ez(sgpu_ctx* c) {
+    SGPU_READY(c);
+    return c->family == 1 && quads_usable(c) ? launch_quad_part(c, 0, 2) : launch_e<kBulk | kCz>(c);
+}
 sgpu_status sgpu_advance_electric_cpml(sgpu_ctx* c) {
     SGPU_READY(c);
-    return c->cpml.on ? launch_e<kCpml | kAll>(c) : SGPU_OK;
+    if (!c->cpml.on) return SGPU_OK;
+    return c->family == 1 && quads_usable(c) ? launch_quad_part(c, 0, 3) : launch_e<kCpml | kAll>(c);
 }
 sgpu_status sgpu_advance_edispersive_e(sgpu_ctx* c) { SGPU_READY(c); return launch_edisp(c); }
 sgpu_status sgpu_advance_mdispersive_h(sgpu_ctx* c) { SGPU_READY(c); return launch_mdisp(c); }
@@ -1954,12 +1964,22 @@ sgpu_status sgpu_advance_nodal_e(sgpu_ctx* c, int n) {
     SGPU_READY(c);
     return launch_sources(c, 0, StepRef{nullptr, n}, kMaskNodal);
 }
-sgpu_status sgpu_advance_hx(sgpu_ctx* c) { SGPU_READY(c); return launch_h<kBulk | kCx>(c); }
-sgpu_status sgpu_advance_hy(sgpu_ctx* c) { SGPU_READY(c); return launch_h<kBulk | kCy>(c); }
-sgpu_status sgpu_advance_hz(sgpu_ctx* c) { SGPU_READY(c); return launch_h<kBulk | kCz>(c); }
+sgpu_status sgpu_advance_hx(sgpu_ctx* c) {
+    SGPU_READY(c);
+    return c->family == 1 && quads_usable(c) ? launch_quad_part(c, 1, 0) : launch_h<kBulk | kCx>(c);
+}
+sgpu_status sgpu_advance_hy(sgpu_ctx* c) {
+    SGPU_READY(c);
+    return c->family == 1 && quads_usable(c) ? launch_quad_part(c, 1, 1) : launch_h<kBulk | kCy>(c);
+}
+sgpu_status sgpu_advance_hz(sgpu_ctx* c) {
+    SGPU_READY(c);
+    return c->family == 1 && quads_usable(c) ? launch_quad_part(c, 1, 2) : launch_h<kBulk | kCz>(c);
+}
 sgpu_status sgpu_advance_magnetic_cpml(sgpu_ctx* c) {
     SGPU_READY(c);
-    return c->cpml.on ? launch_h<kCpml | kAll>(c) : SGPU_OK;
+    if (!c->cpml.on) return SGPU_OK;
+    return c->family == 1 && quads_usable(c) ? launch_quad_part(c, 1, 3) : launch_h<kCpml | kAll>(c);
 }
 sgpu_status sgpu_advance_planewave_h(sgpu_ctx* c, int n) {
     SGPU_READY(c);

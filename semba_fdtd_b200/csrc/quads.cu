@@ -193,6 +193,31 @@ __global__ void __launch_bounds__(kQuadThreads, 8)
     }
 }
 
+// One routine of a half step alone (MODE as quad_march's): one call per routine
+// of 120x110x130 swept cells, 142 us a step with the register-marching kernels,
+// 68 with these.
+template <int SIDE, int MODE>
+__global__ void __launch_bounds__(kQuadThreads, 8)
+    k_quad_part(const __grid_constant__ QuadView g, const __grid_constant__ QuadSide s, int chunk, int bx) {
+    __shared__ float2 tab[256];
+    __shared__ QuadLine zl[kQuadChunk];
+    for (int m = threadIdx.x; m < s.nmed1; m += kQuadThreads) tab[m] = s.tab[m];
+    const int by = blockIdx.x / bx;
+    const int kb = s.z0 + by * chunk, ke = min(kb + chunk, s.z0 + s.nz) - 1;
+    for (int m = threadIdx.x; m <= ke - kb; m += kQuadThreads) zl[m] = s.z[kb + m];
+    int i, j;
+    const bool valid = quad_at(s, (blockIdx.x - by * bx) * kQuadThreads + threadIdx.x, i, j);
+    const QuadX* X = s.x + (i >> 2);
+    const QuadLine Y = ldl(s.y + j);
+    float idx[4];
+    ld4(idx, X->id);
+    const unsigned meet = (MODE & kCpml) && valid ? X->meet & Y.hold : 0u, whole = X->whole;
+    __syncthreads();
+    grid_wait();
+    if ((MODE & kBulk) || __any_sync(0xffffffffu, meet != 0))
+        quad_march<SIDE, (MODE & kCpml) != 0, MODE>(g, s, tab, zl, X, Y, idx, meet, whole, i, j, kb, ke, valid);
+}
+
 __global__ void k_quad_tables(KGrid g, KCpml cp, int nxa, int nya, int nza, int side, QuadX* x, QuadLine* y, QuadLine* z,
                               float2* tab) {
     const int nq = g.pitch / 4, q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -446,6 +471,31 @@ sgpu_status launch_quad(sgpu_ctx* c, int side, StepRef sr, bool sources, const S
                  : launch_after(c->stream, blocks, kQuadThreads, k_quad<0, false>, v, s, g, src, '\0', chunk, bx, blocks);
     }
     return e == cudaSuccess ? SGPU_OK : cuda_error(c, "k_quad", e);
+}
+
+template <int SIDE, int MODE> static cudaError_t launch_part(sgpu_ctx* c) {
+    const QuadSide s = quad_side(c, SIDE);
+    const int bx = (s.threads + kQuadThreads - 1) / kQuadThreads;
+    int chunk = kQuadChunk;
+    while (chunk > 2 && (long long)bx * ((s.nz + chunk - 1) / chunk) < 148 * 16) chunk /= 2;
+    return launch_after(c->stream, bx * ((s.nz + chunk - 1) / chunk), kQuadThreads, k_quad_part<SIDE, MODE>, quad_view(c), s, chunk, bx);
+}
+
+sgpu_status launch_quad_part(sgpu_ctx* c, int side, int what) {
+    const sgpu_status st = quad_prepare(c);
+    if (st) return st;
+    cudaError_t e;
+    switch (4 * side + what) {
+        case 0: e = launch_part<0, kBulk | kCx>(c); break;
+        case 1: e = launch_part<0, kBulk | kCy>(c); break;
+        case 2: e = launch_part<0, kBulk | kCz>(c); break;
+        case 3: e = launch_part<0, kCpml | kAll>(c); break;
+        case 4: e = launch_part<1, kBulk | kCx>(c); break;
+        case 5: e = launch_part<1, kBulk | kCy>(c); break;
+        case 6: e = launch_part<1, kBulk | kCz>(c); break;
+        default: e = launch_part<1, kCpml | kAll>(c); break;
+    }
+    return e == cudaSuccess ? SGPU_OK : cuda_error(c, "k_quad_part", e);
 }
 
 // What steps need on the device before they are captured: a graph holds no

@@ -148,8 +148,9 @@ __device__ __forceinline__ void psi_apply(QuadPsi& s, const float (&pb)[NP], con
 // Advance_H (SIDE 1, :2294-2409) + AdvanceMagneticCPML of the quad at (i, j)
 // over planes kb..ke, in the order of efield_column / hfield_column.  Both
 // sides march so that the z neighbour is the plane before: up on the E side,
-// down on the H side.
-template <int SIDE, bool CP>
+// down on the H side.  MODE (kBulk, kCpml, kCx ..): only the curl, only the
+// corrections, only some components, for the routines called one by one.
+template <int SIDE, bool CP, int MODE = kBulk | kCpml | kAll>
 __device__ __forceinline__ void quad_march(const QuadView& g, const QuadSide& s, const float2* tab, const QuadLine* zl, const QuadX* X, const QuadLine& Y,
                                            const float (&idx)[4], unsigned meet, unsigned whole, int i, int j, int kb, int ke,
                                            bool valid) {
@@ -160,8 +161,8 @@ __device__ __forceinline__ void quad_march(const QuadView& g, const QuadSide& s,
     int c = i + pitch * j + plane * k;
     const int dz = SIDE ? plane : -plane, dy = SIDE ? pitch : -pitch;
     float xk[4], yk[4];  // the other field's x and y components at the plane before
-    ld4(xk, g.F[S] + (c + dz));
-    ld4(yk, g.F[S + 1] + (c + dz));
+    if (MODE & kCy) ld4(xk, g.F[S] + (c + dz));
+    if (MODE & kCx) ld4(yk, g.F[S + 1] + (c + dz));
     unsigned ok0 = 0, ok1 = 0, ok2 = 0;
     if (valid) {
         ok0 = j >= g.sw[O][2] && j <= g.sw[O][3] ? in_range4(i, g.sw[O][0], g.sw[O][1]) : 0u;
@@ -172,19 +173,28 @@ __device__ __forceinline__ void quad_march(const QuadView& g, const QuadSide& s,
 #pragma unroll 1
     for (int n = 0; n < planes; ++n, k += SIDE ? -1 : 1, c -= dz) {
         float x[4], y[4], z[4], xj[4], zj[4], f0[4], f1[4], f2[4];
-        ld4(x, g.F[S] + c);
-        ld4(y, g.F[S + 1] + c);
-        ld4(z, g.F[S + 2] + c);
-        ld4(xj, g.F[S] + (c + dy));
-        ld4(zj, g.F[S + 2] + (c + dy));
-        ld4(f0, g.F[O] + c);
-        ld4(f1, g.F[O + 1] + c);
-        ld4(f2, g.F[O + 2] + c);
-        const float yi = g.F[S + 1][c + (SIDE ? 4 : -1)], zi = g.F[S + 2][c + (SIDE ? 4 : -1)];
-        const unsigned m0 = *(const unsigned*)(g.M8[O] + c), m1 = *(const unsigned*)(g.M8[O + 1] + c),
-                       m2 = *(const unsigned*)(g.M8[O + 2] + c);
         const QuadLine Z = ldl(zl + (k - kb));
         const unsigned live = CP ? meet & Z.hold : 0u;
+        if (!(MODE & kBulk) && !live) continue;  // the carried planes are loaded again below
+        if (MODE & (kCy | kCz)) ld4(x, g.F[S] + c);
+        if (MODE & (kCx | kCz)) ld4(y, g.F[S + 1] + c);
+        if (MODE & (kCx | kCy)) ld4(z, g.F[S + 2] + c);
+        if (MODE & kCz) ld4(xj, g.F[S] + (c + dy));
+        if (MODE & kCx) ld4(zj, g.F[S + 2] + (c + dy));
+        if (MODE & kCx) ld4(f0, g.F[O] + c);
+        if (MODE & kCy) ld4(f1, g.F[O + 1] + c);
+        if (MODE & kCz) ld4(f2, g.F[O + 2] + c);
+        if (!(MODE & kBulk)) {
+            ld4(xk, g.F[S] + (c + dz));
+            ld4(yk, g.F[S + 1] + (c + dz));
+        }
+        float yi = 0.0f, zi = 0.0f;
+        if (MODE & kCz) yi = g.F[S + 1][c + (SIDE ? 4 : -1)];
+        if (MODE & kCy) zi = g.F[S + 2][c + (SIDE ? 4 : -1)];
+        unsigned m0 = 0, m1 = 0, m2 = 0;
+        if (MODE & kCx) m0 = *(const unsigned*)(g.M8[O] + c);
+        if (MODE & kCy) m1 = *(const unsigned*)(g.M8[O + 1] + c);
+        if (MODE & kCz) m2 = *(const unsigned*)(g.M8[O + 2] + c);
         const unsigned on0 = k >= g.sw[O][4] && k <= g.sw[O][5] ? ok0 : 0u;
         const unsigned on1 = k >= g.sw[O + 1][4] && k <= g.sw[O + 1][5] ? ok1 : 0u;
         const unsigned on2 = k >= g.sw[O + 2][4] && k <= g.sw[O + 2][5] ? ok2 : 0u;
@@ -205,13 +215,13 @@ __device__ __forceinline__ void quad_march(const QuadView& g, const QuadSide& s,
         float d1[4], d2[4], v[4];
         float2 t[4];
         const float yb[1] = {Y.pb}, yc[1] = {Y.pc}, zb[1] = {Z.pb}, zc[1] = {Z.pc};
-        {  // x: y derivative of the z component, z derivative of the y component
+        if (MODE & kCx) {  // x: y derivative of the z component, z derivative of the y component
             quad_tab(t, tab, m0);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 d1[e] = dif(z[e], zj[e]);
                 d2[e] = dif(y[e], yk[e]);
-                v[e] = t[e].x * f0[e] + t[e].y * (SIDE ? d2[e] * Z.id - d1[e] * Y.id : d1[e] * Y.id - d2[e] * Z.id);
+                v[e] = !(MODE & kBulk) ? f0[e] : t[e].x * f0[e] + t[e].y * (SIDE ? d2[e] * Z.id - d1[e] * Y.id : d1[e] * Y.id - d2[e] * Z.id);
             }
             if (CP && live) {
                 psi_apply<SIDE == 0>(p0, yb, yc, d1, t, v);
@@ -219,13 +229,13 @@ __device__ __forceinline__ void quad_march(const QuadView& g, const QuadSide& s,
             }
             put4(g.F[O] + c, on0, v, f0);
         }
-        {  // y: z derivative of the x component, x derivative of the z component
+        if (MODE & kCy) {  // y: z derivative of the x component, x derivative of the z component
             quad_tab(t, tab, m1);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 d1[e] = dif(x[e], xk[e]);
                 d2[e] = dif(z[e], nx(z, zi, e));
-                v[e] = t[e].x * f1[e] + t[e].y * (SIDE ? d2[e] * idx[e] - d1[e] * Z.id : d1[e] * Z.id - d2[e] * idx[e]);
+                v[e] = !(MODE & kBulk) ? f1[e] : t[e].x * f1[e] + t[e].y * (SIDE ? d2[e] * idx[e] - d1[e] * Z.id : d1[e] * Z.id - d2[e] * idx[e]);
             }
             if (CP && live) {
                 psi_apply<SIDE == 0>(p2, zb, zc, d1, t, v);
@@ -233,13 +243,13 @@ __device__ __forceinline__ void quad_march(const QuadView& g, const QuadSide& s,
             }
             put4(g.F[O + 1] + c, on1, v, f1);
         }
-        {  // z: x derivative of the y component, y derivative of the x component
+        if (MODE & kCz) {  // z: x derivative of the y component, y derivative of the x component
             quad_tab(t, tab, m2);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 d1[e] = dif(y[e], nx(y, yi, e));
                 d2[e] = dif(x[e], xj[e]);
-                v[e] = t[e].x * f2[e] + t[e].y * (SIDE ? d2[e] * Y.id - d1[e] * idx[e] : d1[e] * idx[e] - d2[e] * Y.id);
+                v[e] = !(MODE & kBulk) ? f2[e] : t[e].x * f2[e] + t[e].y * (SIDE ? d2[e] * Y.id - d1[e] * idx[e] : d1[e] * idx[e] - d2[e] * Y.id);
             }
             if (CP && live) {
                 psi_apply<SIDE == 1>(p4, yb, yc, d2, t, v);

@@ -385,6 +385,8 @@ sgpu_status quad_ready(sgpu_ctx* c);
 // (*applied); with `obs` the observations of that step that read the other
 // field ride along (observers_ride).  launch_observe: those of one side alone.
 sgpu_status launch_quad(sgpu_ctx* c, int side, StepRef sr, bool sources, const StepRef* obs, bool* applied);
+// One routine of the half step alone: components 0..2, or (3) the corrections.
+sgpu_status launch_quad_part(sgpu_ctx* c, int side, int what);
 bool rows_ride(const sgpu_ctx* c, int side);
 bool observers_ride(const sgpu_ctx* c);
 sgpu_status launch_observe(sgpu_ctx* c, int side, StepRef sr);
