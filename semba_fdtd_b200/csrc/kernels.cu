@@ -1082,6 +1082,7 @@ sgpu_status sgpu_init_cpml(sgpu_ctx* c, const sgpu_cpml_desc* d) {
                 any = true;
             }
     k.on = any ? 1 : 0;
+    c->quad_apart = quads_apart(k);
     // psi tensor maps of the TMA kernels: map 9+n of a side is slab bit n
     if (c->tma_ready)
         for (int side = 0; side < 2; ++side)

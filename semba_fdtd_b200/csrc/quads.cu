@@ -268,7 +268,24 @@ size_t table_bytes(const sgpu_ctx* c) {
 
 namespace sgpu {
 
-bool quads_usable(const sgpu_ctx* c) { return tma_usable(c) && c->vol <= kQuadCells && !c->wait_drill && c->quad_mem; }
+// A quad takes one slab of a pair (psi_load).  Grids where some quad meets both,
+// those of two cells in x between two CPML sides, go to the ring or the register
+// kernels, which choose the slab cell by cell.
+bool quads_apart(const KCpml& cp) {
+    for (int f = 0; f < 6 && cp.on; ++f)
+        for (int w = 0; w < 2; ++w) {
+            const Slab &a = cp.s[f][w][0], &b = cp.s[f][w][1];
+            auto meet = [](int alo, int ahi, int blo, int bhi) { return alo <= bhi && blo <= ahi; };
+            if (a.psi && b.psi && meet(a.xlo / 4, a.xhi / 4, b.xlo / 4, b.xhi / 4) && meet(a.ylo, a.yhi, b.ylo, b.yhi) &&
+                meet(a.zlo, a.zhi, b.zlo, b.zhi))
+                return false;
+        }
+    return true;
+}
+
+bool quads_usable(const sgpu_ctx* c) {
+    return tma_usable(c) && c->vol <= kQuadCells && c->quad_apart && !c->wait_drill && c->quad_mem;
+}
 
 QuadView quad_view(const sgpu_ctx* c) {
     QuadView v{};

@@ -107,7 +107,7 @@ __device__ __forceinline__ void quad_tab(float2 (&t)[4], const float2* tab, unsi
     }
 }
 // The old psi of one correction of a quad: slab pair N, N + 1, whose live bits
-// are in `live`.  Loaded with the plane's fields, before any store of the
+// (at most one: quads_apart) are in `live`.  Loaded with the plane's fields, before any store of the
 // plane: a load behind a store would wait for memory once per correction.
 struct QuadPsi {
     float v[4];

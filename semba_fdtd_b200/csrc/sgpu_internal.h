@@ -311,6 +311,7 @@ struct sgpu_ctx {
     // tables of the quad kernels (quads.cu): one x table and two line tables a side
     void* quad_mem = nullptr;
     bool quad_ok = false;
+    bool quad_apart = true;  // no quad of x cells meets both slabs of a CPML pair
     // ... and the source rows by warp and plane (quad_src_fits: every row lies on
     // a cell the kernels update)
     sgpu::SrcRows src_rows[2];
@@ -379,6 +380,7 @@ void ctx_free(sgpu_ctx* c, void* p);
 // The curl + CPML half step of quads.cu (0 E, 1 H), its tables, and whether the
 // default kernel family takes it for this context.
 bool quads_usable(const sgpu_ctx* c);
+bool quads_apart(const KCpml& cp);
 sgpu_status quad_alloc(sgpu_ctx* c);
 sgpu_status quad_ready(sgpu_ctx* c);
 // With `sources` the source rows of step sr are applied too when they can be

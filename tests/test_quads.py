@@ -49,6 +49,33 @@ def test_ragged_quads_equal_the_oracle(n, layers, boundary):
             assert_bits_equal(s.field(c), o.field(c), err_msg=f"component {c}")
 
 
+@pytest.mark.parametrize("mode", ["graph", "fused", "routines", "batch"])
+@pytest.mark.parametrize("layers", [4, 8, 12])
+def test_both_x_slabs_in_one_quad_equal_the_oracle(layers, mode):
+    """Two cells in x: the low slab of Hy and Hz ends on the first cell of a
+    quad and the high slab begins on its last, as nowhere else in a grid the
+    set-up makes."""
+    from semba_fdtd_b200.batch import Batch
+    pb, _ = _case((2, 7, 6), layers)
+    o = oracle.Oracle(pb)
+    want = o.step(pb.nsteps + 1)
+    with Solver(pb) as s:
+        x0 = s.alloc[0][0]
+        for c in (4, 5):
+            assert (s.sinpml[c][0] - 1 - x0) // 4 == (s.sinpml[c][1] + 1 - x0) // 4
+        if mode != "batch":
+            assert_bits_equal(s.run(mode=mode), want)
+            got = [s.field(c) for c in range(6)]
+    if mode == "batch":
+        with Batch(64 << 20, 2) as b:
+            slot = b.add(pb)
+            b.run_all()
+            assert_bits_equal(b.probes(slot), want)
+            got = [b.field(slot, c) for c in range(6)]
+    for c in range(6):
+        assert_bits_equal(got[c], o.field(c), err_msg=f"component {c}")
+
+
 @pytest.mark.parametrize("inset", [2, 5, 9])
 def test_rows_and_observers_in_the_half_steps(inset):
     """A TF/SF box from one that fills the grid (source rows by k_sources) to a
