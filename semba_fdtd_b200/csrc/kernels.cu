@@ -1417,7 +1417,9 @@ sgpu_status build_sources(sgpu_ctx* c) {
         k.h_first = c->h_first;
         k.pw_only = 1;
         for (const SrcEntry& en : ent) k.pw_only &= en.type == kSrcPlaneWave;
-        if (!c->arena && quads_usable(c) && rows_ride(c, side)) {
+        // kept wherever the quad kernels may come to serve this context: it may
+        // list its rows under the wait drill and step without it
+        if (!c->arena && c->quad_mem && rows_ride(c, side)) {
             SrcRows& h = c->src_rows[side];
             h.first.reserve(rnode.size());
             for (size_t r = 0; r < rnode.size(); ++r) h.first.push_back(ent[rptr[r]]);
@@ -2207,8 +2209,8 @@ sgpu_status sgpu_kernels_per_step(const sgpu_ctx* c, int* n) {
     const bool quads = c->family == 1 && quads_usable(c), ride = quads && observers_ride(c);
     for (const KDisp* d : {c->disp_on ? &c->disp : nullptr, c->mdisp_on ? &c->mdisp : nullptr})
         if (d) k += d->n[0] + d->n[1] + d->n[2] <= kAdeTogether ? 1 : (d->n[0] > 0) + (d->n[1] > 0) + (d->n[2] > 0);
-    k += c->src[0].nrows > 0 && !(quads && !c->disp_on && c->quad_src_fits && rows_ride(c, 0));
-    k += c->src[1].nrows > 0 && !(quads && !c->mdisp_on && c->quad_src_fits && rows_ride(c, 1));
+    k += c->src[0].nrows > 0 && !(quads && !c->disp_on && rows_grouped(c, 0));
+    k += c->src[1].nrows > 0 && !(quads && !c->mdisp_on && rows_grouped(c, 1));
     if (!ride) k += (c->probes.n > 0) + (int)c->vprobes.size();
     k += c->border.cl_cells > 0;
     k += c->border.mur_cells > 0;

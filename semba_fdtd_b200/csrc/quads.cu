@@ -368,27 +368,29 @@ QuadSide quad_side(const sgpu_ctx* c, int side) {
 }
 
 // The source rows grouped by (warp's quads, plane) of their node, in the
-// kernel's numbering of the quads.
+// kernel's numbering of the quads.  A side whose rows were not kept for this
+// (src_rows), or of which one lies on no cell the side's kernel updates, gets no
+// groups, and k_sources applies its rows.
 static sgpu_status quad_sources(sgpu_ctx* c) {
     if (c->quad_src_ok) return SGPU_OK;
     for (void* q : c->quad_src_allocs) ctx_free(c, q);
     c->quad_src_allocs.clear();
-    c->quad_src_fits = true;
-    for (int side = 0; side < 2; ++side) {  // src_rows holds a side's rows where rows_ride
+    for (int side = 0; side < 2; ++side) {
         c->quad_sptr[side] = nullptr;
         c->quad_srow[side] = nullptr;
         const SrcRows& h = c->src_rows[side];
         const size_t n = h.node.size();
-        if (n == 0 || !c->quad_src_fits) continue;
+        if (n == 0 || n != (size_t)c->src[side].nrows) continue;
         const QuadSide s = quad_side(c, side);
         const int we = s.xlo + s.xhi, wi = s.nq - we;
         const size_t keys = (size_t)((s.threads + 31) / 32) * s.nz;
         std::vector<int> ptr(keys + 1, 0), key(n);
+        bool fits = true;
         for (size_t r = 0; r < n; ++r) {
             const int q = h.node[r] % c->pitch / 4, j = (int)(h.node[r] % c->plane) / c->pitch - s.y0,
                       k = (int)(h.node[r] / c->plane) - s.z0;
             if (h.comp[r] / 3 != side || q >= s.nq || j < 0 || j >= s.ny || k < 0 || k >= s.nz) {
-                c->quad_src_fits = false;  // no thread of the side updates this cell
+                fits = false;  // no thread of the side updates this cell
                 break;
             }
             const bool in = q >= s.xlo && q < s.nq - s.xhi;
@@ -396,7 +398,7 @@ static sgpu_status quad_sources(sgpu_ctx* c) {
             key[r] = p / 32 * s.nz + k;
             ++ptr[key[r] + 1];
         }
-        if (!c->quad_src_fits) continue;
+        if (!fits) continue;
         for (size_t q = 0; q < keys; ++q) ptr[q + 1] += ptr[q];
         std::vector<int> at(ptr.begin(), ptr.end() - 1);
         std::vector<QuadRow> row(n);
@@ -422,6 +424,8 @@ bool rows_ride(const sgpu_ctx* c, int side) {
     const QuadSide s = quad_side(c, side);
     return kCellsARow * c->src[side].nrows <= 4ll * s.nq * s.ny * s.nz;
 }
+
+bool rows_grouped(const sgpu_ctx* c, int side) { return c->quad_src_ok && c->quad_sptr[side]; }
 
 bool observers_ride(const sgpu_ctx* c) { return (int)c->vprobes.size() <= kQuadVol && c->farfields.size() <= 1; }
 
@@ -468,9 +472,9 @@ sgpu_status launch_quad(sgpu_ctx* c, int side, StepRef sr, bool sources, const S
     const QuadView v = quad_view(c);
     const KGrid g = kgrid(c);
     QuadSrc src{};
-    if (sources && rows_ride(c, side)) {
+    if (sources && c->src[side].nrows) {
         if ((st = quad_sources(c))) return st;
-        if (c->quad_src_fits) {
+        if (rows_grouped(c, side)) {
             src = QuadSrc{c->quad_sptr[side], (const QuadRow*)c->quad_srow[side], c->src[side], c->d_tiempo, c->t_n0, c->dt, sr};
             *applied = true;
         }

@@ -312,13 +312,13 @@ struct sgpu_ctx {
     void* quad_mem = nullptr;
     bool quad_ok = false;
     bool quad_apart = true;  // no quad of x cells meets both slabs of a CPML pair
-    // ... and the source rows by warp and plane (quad_src_fits: every row lies on
-    // a cell the kernels update)
+    // ... and a side's source rows by warp and plane (none where quad_sptr is
+    // null: the rows are k_sources' then)
     sgpu::SrcRows src_rows[2];
     int* quad_sptr[2] = {};
     void* quad_srow[2] = {};
     std::vector<void*> quad_src_allocs;
-    bool quad_src_ok = false, quad_src_fits = false;
+    bool quad_src_ok = false;
     // scratch
     unsigned int* d_flag = nullptr;
     // TMA-pipelined fused kernels: tensor maps and the bounded-wait error word
@@ -389,7 +389,8 @@ sgpu_status quad_ready(sgpu_ctx* c);
 sgpu_status launch_quad(sgpu_ctx* c, int side, StepRef sr, bool sources, const StepRef* obs, bool* applied);
 // One routine of the half step alone: components 0..2, or (3) the corrections.
 sgpu_status launch_quad_part(sgpu_ctx* c, int side, int what);
-bool rows_ride(const sgpu_ctx* c, int side);
+bool rows_ride(const sgpu_ctx* c, int side);     // few enough to, where the kernels run
+bool rows_grouped(const sgpu_ctx* c, int side);  // and they do
 bool observers_ride(const sgpu_ctx* c);
 sgpu_status launch_observe(sgpu_ctx* c, int side, StepRef sr);
 struct FarArgs;

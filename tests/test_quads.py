@@ -154,3 +154,42 @@ def test_batch_of_small_and_large_instances():
         b.run_all()
         for s, w in zip(slots, want):
             assert_bits_equal(b.probes(s), w)
+
+
+@pytest.mark.parametrize("mode", ["graph", "fused"])
+def test_sources_listed_while_the_ring_served(mode):
+    """The source rows are listed under the wait drill, which keeps the quads
+    off, and the steps run after it."""
+    pb, _ = _case((41, 26, 23), 3, steps=70)
+    o = oracle.Oracle(pb)
+    with Solver(pb) as s:
+        h = s.handle
+        s._check(s.lib.sgpu_set_wait_drill(h, 1))
+        s._check(s.lib.sgpu_advance_nodal_e(h, 0))  # lists the rows; no half step, so no wait runs out
+        s._check(s.lib.sgpu_set_wait_drill(h, 0))
+        for c in range(6):
+            s.upload_field(c, np.zeros(s.field_shape(c), np.float32))
+        assert_bits_equal(s.run(mode=mode), o.step(pb.nsteps + 1))
+        for c in range(6):
+            assert_bits_equal(s.field(c), o.field(c), err_msg=f"component {c}")
+
+
+@pytest.mark.parametrize("calls", ["halves", "steps"])
+def test_sources_of_an_instance_stepped_by_its_context(calls):
+    """sgpu_batch_instance hands out a context; stepping it applies the sources."""
+    import ctypes as C
+    from semba_fdtd_b200.batch import Batch
+    pb, _ = _case((41, 26, 23), 3, steps=36)
+    o = oracle.Oracle(pb)
+    o.step(pb.nsteps + 1)
+    with Batch(256 << 20, 2) as b:
+        slot, ctx = b.add(pb), C.c_void_p()
+        b._check(b.lib.sgpu_batch_instance(b._h, slot, C.byref(ctx)), "instance")
+        if calls == "steps":
+            assert b.lib.sgpu_advance_steps(ctx, 0, pb.nsteps + 1) == 0
+        for n in range(pb.nsteps + 1 if calls == "halves" else 0):
+            assert b.lib.sgpu_advance_e(ctx, n) == 0
+            assert b.lib.sgpu_advance_h(ctx, n) == 0
+        assert b.lib.sgpu_synchronize(ctx) == 0
+        for c in range(6):
+            assert_bits_equal(b.field(slot, c), o.field(c), err_msg=f"component {c}")
