@@ -1039,6 +1039,7 @@ sgpu_status sgpu_init_cpml(sgpu_ctx* c, const sgpu_cpml_desc* d) {
     if (!c || !d) return set_error(c, SGPU_ERR_ARG, "null cpml descriptor");
     free_list(c, c->cpml_allocs);
     c->quad_ok = false;
+    c->quad_src_ok = false;  // the slabs decide the quads' numbering
     KCpml& k = c->cpml;
     k = KCpml{};
     sgpu_status s;

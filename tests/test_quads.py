@@ -2,6 +2,7 @@
 around multiples of four and of the 32-cell pitch, CPML slabs that begin and
 end inside a quad, both sides of an axis in one quad, grids of one block and
 a few planes, and both sides of the line to the TMA ring."""
+import ctypes
 import tempfile
 from dataclasses import replace
 from pathlib import Path
@@ -11,7 +12,7 @@ import pytest
 
 import oracle
 from bits import assert_bits_equal
-from semba_fdtd_b200 import Solver, casegen, read_case
+from semba_fdtd_b200 import Solver, _lib, casegen, read_case
 
 pytestmark = pytest.mark.gpu
 _DIR = Path(tempfile.mkdtemp(prefix="semba_quads_"))
@@ -177,14 +178,13 @@ def test_sources_listed_while_the_ring_served(mode):
 @pytest.mark.parametrize("calls", ["halves", "steps"])
 def test_sources_of_an_instance_stepped_by_its_context(calls):
     """sgpu_batch_instance hands out a context; stepping it applies the sources."""
-    import ctypes as C
     from semba_fdtd_b200.batch import Batch
     pb, _ = _case((41, 26, 23), 3, steps=36)
     o = oracle.Oracle(pb)
     o.step(pb.nsteps + 1)
     with Batch(256 << 20, 2) as b:
-        slot, ctx = b.add(pb), C.c_void_p()
-        b._check(b.lib.sgpu_batch_instance(b._h, slot, C.byref(ctx)), "instance")
+        slot, ctx = b.add(pb), ctypes.c_void_p()
+        b._check(b.lib.sgpu_batch_instance(b._h, slot, ctypes.byref(ctx)), "instance")
         if calls == "steps":
             assert b.lib.sgpu_advance_steps(ctx, 0, pb.nsteps + 1) == 0
         for n in range(pb.nsteps + 1 if calls == "halves" else 0):
@@ -193,3 +193,54 @@ def test_sources_of_an_instance_stepped_by_its_context(calls):
         assert b.lib.sgpu_synchronize(ctx) == 0
         for c in range(6):
             assert_bits_equal(b.field(slot, c), o.field(c), err_msg=f"component {c}")
+
+
+def _new_cpml(s, kind):
+    """sgpu_init_cpml of a stepping context: the problem's y and z slabs with x
+    slabs of other widths, or none at all; coefficients of the usual size."""
+    class Desc(ctypes.Structure):
+        _fields_ = [("pmlc", (_lib.Lim * 6) * 6)] + [(n, _lib.c_float_p * 3) for n in ("be", "ce", "bm", "cm")]
+
+    d, rng, keep = Desc(), np.random.default_rng(7), []
+    widths = {"none": (0, 0), "thin": (1, 2), "wide": (9, 6)}[kind]
+    for f in range(6):
+        w, q = s.sweep[f], s.sinpml[f]
+        boxes = [(*w[:4], w[4], q[4] - 1), (*w[:4], q[5] + 1, w[5]), (*w[:2], w[2], q[2] - 1, *w[4:]),
+                 (*w[:2], q[3] + 1, w[3], *w[4:]), (w[0], w[0] + widths[0] - 1, *w[2:]), (w[1] - widths[1] + 1, w[1], *w[2:])]
+        for r, b in enumerate(boxes):
+            d.pmlc[f][r] = _lib.Lim(*((1, 0, 1, 0, 1, 0) if kind == "none" else b))
+    for a, c in enumerate((3, 4, 5)):
+        n = s.alloc[c][2 * a + 1] - s.alloc[c][2 * a] + 1
+        for name, lo, hi in (("be", 0.3, 0.9), ("ce", -100, 0), ("bm", 0.3, 0.9), ("cm", -100, 0)):
+            v = rng.uniform(lo, hi, n).astype(np.float32)
+            keep.append(v)
+            getattr(d, name)[a] = v.ctypes.data_as(_lib.c_float_p)
+    s._check(s.lib.sgpu_init_cpml(s.handle, ctypes.byref(d)), "sgpu_init_cpml")
+
+
+@pytest.mark.parametrize("mode", ["graph", "fused"])
+@pytest.mark.parametrize("kind", ["none", "thin", "wide"])
+def test_cpml_set_again_between_steps(kind, mode):
+    """The slabs decide how quads are numbered, and so the groups of the source
+    rows; the register-marching kernels, which number nothing, are the reference."""
+    n = (61, 31, 29)
+    b = casegen._Builder(n, 60, 5)
+    b.steps([0.003], [0.003], [0.003])
+    ds = casegen.courant_dt(0.003) / 2
+    b.planewave([11] * 3, [v - 11 for v in n], 0.7, 1.9, 1.1, 0.4, "gauss.exc", ds,
+                casegen.gaussian(ds, 20e-12, 60e-12, 0.2e-9))
+    b.probe("p", "electric", [v // 2 for v in n], "xyz")
+    pb = read_case(b.write(_DIR, "cpml_again"))
+    out = []
+    for family in (1, 0):
+        with Solver(pb, kernel_family=family) as s:
+            s.step(20, mode=mode)
+            _new_cpml(s, kind)
+            s.step(41, mode=mode)
+            out.append([s.probes()] + [s.field(c) for c in range(6)])
+            k = ctypes.c_int()
+            s._check(s.lib.sgpu_kernels_per_step(s.handle, ctypes.byref(k)))
+            assert k.value == (2 if family else 5)  # the rows ride; the probes, too, where they are the quads'
+    assert np.isfinite(out[0][1]).all() and np.abs(out[0][1]).max() > 0
+    for a, w in zip(*out):
+        assert_bits_equal(a, w)
