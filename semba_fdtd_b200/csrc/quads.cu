@@ -218,9 +218,12 @@ __global__ void __launch_bounds__(kQuadThreads, 8)
         quad_march<SIDE, (MODE & kCpml) != 0, MODE>(g, s, tab, zl, X, Y, idx, meet, whole, i, j, kb, ke, valid);
 }
 
-__global__ void k_quad_tables(KGrid g, KCpml cp, int nxa, int nya, int nza, int side, QuadX* x, QuadLine* y, QuadLine* z,
-                              float2* tab) {
-    const int nq = g.pitch / 4, q = blockIdx.x * blockDim.x + threadIdx.x;
+// Side blockIdx.y's tables, `one` bytes a side (table_bytes).
+__global__ void k_quad_tables(KGrid g, KCpml cp, int nxa, int nya, int nza, char* mem, size_t one) {
+    const int side = blockIdx.y, nq = g.pitch / 4, q = blockIdx.x * blockDim.x + threadIdx.x;
+    QuadX* const x = (QuadX*)(mem + side * one);
+    QuadLine *const y = (QuadLine*)(x + nq), *const z = y + nya;
+    float2* const tab = (float2*)(z + nza);
     for (int m = q; m < g.nmed1; m += gridDim.x * blockDim.x)
         tab[m] = side ? make_float2(g.gm1[m], g.gm2[m]) : make_float2(g.g1[m], g.g2[m]);
     if (q >= nq + nya + nza) return;
@@ -254,6 +257,10 @@ __global__ void k_quad_tables(KGrid g, KCpml cp, int nxa, int nya, int nza, int 
         (ax == 1 ? y : z)[at] = r;
     }
 }
+
+// Launched plainly after the tables: it begins when they are complete and
+// visible, so the quad kernel that follows it may read them before grid_wait.
+__global__ void k_tables_done() {}
 
 sgpu_status cuda_error(sgpu_ctx* c, const char* what, cudaError_t e) {
     return set_error(c, SGPU_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
@@ -318,16 +325,12 @@ sgpu_status quad_alloc(sgpu_ctx* c) {
 // The tables are built on first use and again after sgpu_init_cpml.
 sgpu_status quad_prepare(sgpu_ctx* c) {
     if (c->quad_ok) return SGPU_OK;
-    const size_t nx = c->pitch / 4, one = table_bytes(c);
-    for (int h = 0; h < 2; ++h) {
-        QuadX* x = (QuadX*)((char*)c->quad_mem + h * one);
-        QuadLine* y = (QuadLine*)(x + nx);
-        const int n = (int)nx + c->nya + c->nza;
-        k_quad_tables<<<(n + 127) / 128, 128, 0, c->stream>>>(kgrid(c), c->cpml, c->nxa, c->nya, c->nza, h, x, y, y + c->nya,
-                                                         (float2*)(y + c->nya + c->nza));
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return cuda_error(c, "k_quad_tables", e);
-    }
+    const int n = c->pitch / 4 + c->nya + c->nza;
+    k_quad_tables<<<dim3((n + 127) / 128, 2), 128, 0, c->stream>>>(kgrid(c), c->cpml, c->nxa, c->nya, c->nza, (char*)c->quad_mem,
+                                                                   table_bytes(c));
+    k_tables_done<<<1, 1, 0, c->stream>>>();
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_error(c, "k_quad_tables", e);
     c->quad_ok = true;
     return SGPU_OK;
 }

@@ -344,7 +344,9 @@ namespace sgpu {
 // its predecessor still runs: all its threads must call grid_wait (which
 // returns once the predecessor has finished and its writes are visible) before
 // they touch anything a kernel of the step writes, and before any of them
-// returns.  grid_wait also lets the kernel's own successor be scheduled.
+// returns.  grid_wait also lets the kernel's own successor be scheduled.  What a
+// kernel reads before grid_wait must come from further back than its
+// predecessor: only after the wait are the predecessor's writes visible.
 #ifdef __CUDACC__
 __device__ __forceinline__ void grid_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");

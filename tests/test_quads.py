@@ -244,3 +244,23 @@ def test_cpml_set_again_between_steps(kind, mode):
     assert np.isfinite(out[0][1]).all() and np.abs(out[0][1]).max() > 0
     for a, w in zip(*out):
         assert_bits_equal(a, w)
+
+
+@pytest.mark.parametrize("first", ["sgpu_advance_h", "sgpu_advance_hx", "sgpu_advance_hz", "sgpu_advance_magnetic_cpml"])
+@pytest.mark.parametrize("n,layers", [((5, 6, 7), 1), ((61, 40, 37), 5)])
+def test_a_context_that_begins_with_h(n, layers, first):
+    """The first quad kernel of a context follows the kernel that makes its
+    tables, and reads them before it waits; the register-marching kernels, which
+    have no tables, are the reference."""
+    pb, _ = _case(n, layers)
+    out = []
+    for family in (1, 0):
+        rng = np.random.default_rng(3)
+        with Solver(pb, kernel_family=family) as s:
+            for c in range(6):
+                s.upload_field(c, rng.standard_normal(s.field_shape(c)).astype(np.float32))
+            call = getattr(s.lib, first)
+            s._check(call(s.handle, 0) if first == "sgpu_advance_h" else call(s.handle), first)
+            out.append([s.field(c) for c in range(6)])
+    for c, (a, w) in enumerate(zip(*out)):
+        assert_bits_equal(a, w, err_msg=f"component {c}")
