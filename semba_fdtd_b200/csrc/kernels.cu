@@ -702,8 +702,7 @@ void keep_pool_memory(int device) {
     done[device] = true;
 }
 
-void* dev_malloc(sgpu_ctx* c, size_t bytes) {
-    if (c->arena) return arena_alloc(c->arena, bytes);
+void* pool_malloc(sgpu_ctx* c, size_t bytes) {
     keep_pool_memory(c->device);
     void* p = nullptr;
     if (cudaMallocAsync(&p, bytes, c->stream) == cudaSuccess) return p;
@@ -716,6 +715,8 @@ void* dev_malloc(sgpu_ctx* c, size_t bytes) {
     cudaGetLastError();
     return nullptr;
 }
+
+void* dev_malloc(sgpu_ctx* c, size_t bytes) { return c->arena ? arena_alloc(c->arena, bytes) : pool_malloc(c, bytes); }
 
 void dev_free(sgpu_ctx* c, void* p) {
     if (!p) return;
@@ -844,7 +845,7 @@ sgpu_status sgpu::create_in(const sgpu_grid_desc* d, Arena* arena, cudaStream_t 
     if ((s = dalloc(c, &c->d_flag, 1))) return fail(s);
     if ((s = dalloc(c, &c->d_err, 1))) return fail(s);
     CUDA_TRY(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-    if ((s = quad_alloc(c))) return fail(s);
+    quad_alloc(c);
     c->tma_ready = build_tensor_maps(c);
     if (c->tma_ready) {
         const int smax = (int)(kTmaSmem + 2 * kShTable * sizeof(float));
@@ -889,8 +890,7 @@ void sgpu_destroy(sgpu_ctx* c) {
     free_list(c, c->probe_allocs);
     free_list(c, c->vprobe_allocs);
     free_farfields(c);
-    if (c->quad_mem && c->arena) cudaFreeAsync(c->quad_mem, c->stream);
-    else dev_free(c, c->quad_mem);
+    if (c->quad_mem) cudaFreeAsync(c->quad_mem, c->stream);
     free_list(c, c->quad_src_allocs);
     if (c->stream && c->own_stream) cudaStreamDestroy(c->stream);
     if (c->host && c->host_free) c->host_free(c->host);
@@ -1011,6 +1011,7 @@ sgpu_status sgpu::narrow_media(sgpu_ctx* c, int comp) {
 }
 
 void* sgpu::ctx_malloc(sgpu_ctx* c, size_t bytes) { return dev_malloc(c, bytes); }
+void* sgpu::ctx_pool_malloc(sgpu_ctx* c, size_t bytes) { return pool_malloc(c, bytes); }
 void sgpu::ctx_free(sgpu_ctx* c, void* p) { dev_free(c, p); }
 bool sgpu::tma_usable(const sgpu_ctx* c) { return c->tma_ready && c->num_media < 256; }
 void sgpu::keep_device_pool(int device) { keep_pool_memory(device); }

@@ -310,16 +310,9 @@ QuadView quad_view(const sgpu_ctx* c) {
 // Room for the tables, taken with the context's other buffers, so that a
 // context set up after another finds the pool's free blocks whole.  In a batch,
 // too, from the device's pool: the arena holds what an instance's footprint
-// counts.
-sgpu_status quad_alloc(sgpu_ctx* c) {
-    if (c->vol > kQuadCells) return SGPU_OK;
-    const size_t bytes = 2 * table_bytes(c);
-    if (!c->arena) c->quad_mem = ctx_malloc(c, bytes);
-    else if (cudaMallocAsync(&c->quad_mem, bytes, c->stream) != cudaSuccess) {
-        cudaGetLastError();
-        c->quad_mem = nullptr;
-    }
-    return c->quad_mem ? SGPU_OK : set_error(c, SGPU_ERR_OOM, "quad tables");
+// counts.  Where the pool has none left the ring serves the context.
+void quad_alloc(sgpu_ctx* c) {
+    if (c->vol <= kQuadCells) c->quad_mem = ctx_pool_malloc(c, 2 * table_bytes(c));
 }
 
 // The tables are built on first use and again after sgpu_init_cpml.
@@ -411,7 +404,7 @@ static sgpu_status quad_sources(sgpu_ctx* c) {
         if (dp) c->quad_src_allocs.push_back(dp);
         void* dr = ctx_malloc(c, n * sizeof(QuadRow));
         if (dr) c->quad_src_allocs.push_back(dr);
-        if (!dp || !dr) return set_error(c, SGPU_ERR_OOM, "source rows by warp");
+        if (!dp || !dr) continue;  // no room for groups: the rows stay with k_sources
         cudaError_t e = cudaMemcpyAsync(dp, ptr.data(), ptr.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(dr, row.data(), n * sizeof(QuadRow), cudaMemcpyHostToDevice, c->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);

@@ -379,11 +379,13 @@ sgpu_status host_create_in(const sgpu_problem* p, sgpu_ctx* plan, int max_steps,
 // Device memory of a context (the batch's arena or the device's pool).
 void* ctx_malloc(sgpu_ctx* c, size_t bytes);
 void ctx_free(sgpu_ctx* c, void* p);
+// From the device's pool also for a context in an arena; cudaFreeAsync returns it.
+void* ctx_pool_malloc(sgpu_ctx* c, size_t bytes);
 // The curl + CPML half step of quads.cu (0 E, 1 H), its tables, and whether the
 // default kernel family takes it for this context.
 bool quads_usable(const sgpu_ctx* c);
 bool quads_apart(const KCpml& cp);
-sgpu_status quad_alloc(sgpu_ctx* c);
+void quad_alloc(sgpu_ctx* c);
 sgpu_status quad_ready(sgpu_ctx* c);
 // With `sources` the source rows of step sr are applied too when they can be
 // (*applied); with `obs` the observations of that step that read the other

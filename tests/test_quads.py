@@ -264,3 +264,48 @@ def test_a_context_that_begins_with_h(n, layers, first):
             out.append([s.field(c) for c in range(6)])
     for c, (a, w) in enumerate(zip(*out)):
         assert_bits_equal(a, w, err_msg=f"component {c}")
+
+
+def test_an_instance_without_room_for_its_tables():
+    """The quad tables of a batch's instance come from the device's memory pool,
+    not the arena: where the pool refuses them the ring serves the instance."""
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    from semba_fdtd_b200.batch import Batch
+
+    def ok(r):
+        assert int(r[0]) == 0, r
+        return r[1] if len(r) == 2 else None
+
+    pb, _ = _case((41, 26, 23), 3)
+    o = oracle.Oracle(pb)
+    want = o.step(pb.nsteps + 1)
+    with Batch(64 << 20, 2) as b:
+        full, taken = rt.cudaMemPoolProps(), []
+        full.allocType = rt.cudaMemAllocationType.cudaMemAllocationTypePinned
+        full.location.type = rt.cudaMemLocationType.cudaMemLocationTypeDevice
+        full.maxSize = 2 << 20
+        default, full = ok(rt.cudaDeviceGetDefaultMemPool(0)), ok(rt.cudaMemPoolCreate(full))
+        for size in (1 << 20, 1 << 12):
+            while True:
+                err, p = rt.cudaMallocFromPoolAsync(size, full, rt.cudaStream_t(0))
+                if int(err):
+                    break
+                taken.append(p)
+                assert len(taken) < 1 << 12, "the pool is not bounded"
+        ok(rt.cudaDeviceSetMemPool(0, full))
+        try:
+            slot = b.add(pb)
+        finally:
+            ok(rt.cudaDeviceSetMemPool(0, default))
+            for p in taken:
+                ok(rt.cudaFreeAsync(p, rt.cudaStream_t(0)))
+            ok(rt.cudaStreamSynchronize(rt.cudaStream_t(0)))
+            ok(rt.cudaMemPoolDestroy(full))
+        ctx, k = ctypes.c_void_p(), ctypes.c_int()
+        b._check(b.lib.sgpu_batch_instance(b._h, slot, ctypes.byref(ctx)), "instance")
+        assert b.lib.sgpu_kernels_per_step(ctx, ctypes.byref(k)) == 0
+        assert k.value == 4  # E, H, sources and probes: with the quads the probes ride
+        b.run_all()
+        assert_bits_equal(b.probes(slot), want)
+        for c in range(6):
+            assert_bits_equal(b.field(slot, c), o.field(c), err_msg=f"component {c}")
