@@ -542,12 +542,14 @@ sgpu_status sgpu_farfield_transform(sgpu_ctx* c, int id, const sgpu_farfield_ang
     double2* d_dft = nullptr;
     double* d_rows = nullptr;
     const int nc = (int)cells.size(), nd = (int)dirs.size();
-    cudaError_t e = cudaMallocAsync(&d_cells, sizeof(TCell) * nc, c->stream);
-    if (e == cudaSuccess) e = cudaMallocAsync(&d_cur, sizeof(Currents) * (size_t)nc * F.nf, c->stream);
-    if (e == cudaSuccess) e = cudaMallocAsync(&d_dirs, sizeof(Dir) * nd, c->stream);
-    if (e == cudaSuccess) e = cudaMallocAsync(&d_freq, sizeof(float) * F.nf, c->stream);
-    if (e == cudaSuccess) e = cudaMallocAsync(&d_dft, sizeof(double2) * F.nf, c->stream);
-    if (e == cudaSuccess) e = cudaMallocAsync(&d_rows, sizeof(double) * 9 * (size_t)need, c->stream);
+    auto take = [&](auto*& p, size_t n) {
+        p = (std::decay_t<decltype(p)>)ctx_pool_malloc(c, sizeof(*p) * n);
+        return p != nullptr;
+    };
+    cudaError_t e = take(d_cells, nc) && take(d_cur, (size_t)nc * F.nf) && take(d_dirs, nd) && take(d_freq, F.nf) &&
+                            take(d_dft, F.nf) && take(d_rows, 9 * (size_t)need)
+                        ? cudaSuccess
+                        : cudaErrorMemoryAllocation;
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_cells, cells.data(), sizeof(TCell) * nc, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_dirs, dirs.data(), sizeof(Dir) * nd, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_freq, F.freq.data(), sizeof(float) * F.nf, cudaMemcpyHostToDevice, c->stream);
