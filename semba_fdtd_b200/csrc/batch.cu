@@ -128,6 +128,11 @@ struct InstDesc {
 struct FieldItem {
     int slot, ib, jb, kb, ke, cp;
 };
+// The quad items of one instance and side: `groups` of 64 quads by planes
+// z0..z0+nz-1 in chunks, from item `first` of the list on.
+struct QuadRun {
+    int slot, first, groups, z0, nz;
+};
 struct RangeItem {
     int slot, sub;     // sub: E component (ADE) or side (sources)
     long long q0, q1;  // node / row / probe range
@@ -215,8 +220,8 @@ struct QuadInst {
 };
 static_assert(sizeof(QuadView) % 4 == 0 && sizeof(QuadSide) % 4 == 0, "copied by words");
 // Planes an item: 4, 8, 16, 32 took 956, 1004, 1074, 1265 us a step (24
-// instances, 42 M swept cells; the ring 1284); at 8 the host's lists are half
-// as long as at 4.
+// instances, 42 M swept cells; the ring 1284); at 8 the lists are half as long
+// as at 4.
 constexpr int kBatchQuadThreads = 64, kBatchQuadChunk = 8, kBatchQuadBlocks = 8;
 template <int SIDE>
 __global__ void __launch_bounds__(kBatchQuadThreads, kBatchQuadBlocks)
@@ -255,6 +260,20 @@ __global__ void __launch_bounds__(kBatchQuadThreads, kBatchQuadBlocks)
         __syncthreads();
         if (__any_sync(0xffffffffu, meet != 0)) quad_march<SIDE, true>(v, s, tab, zl, X, Y, idx, meet, whole, i, j, w.kb, w.ke, valid);
         else quad_march<SIDE, false>(v, s, tab, zl, X, Y, idx, meet, whole, i, j, w.kb, w.ke, valid);
+    }
+}
+
+// The items of every run, written out on the device (blockIdx.x a run).  The host
+// sends 20 bytes an instance: the items of 24 instances of 160 cells an edge are
+// 1.7 MB a side, and the first advance after a join took the host 1940 us with
+// lists made there, 560 us so (720 us with the ring's lists of larger items).
+__global__ void k_quad_items(const QuadRun* __restrict__ runs, FieldItem* items) {
+    const QuadRun r = runs[blockIdx.x];
+    const int n = r.groups * ((r.nz + kBatchQuadChunk - 1) / kBatchQuadChunk);
+    for (int q = blockIdx.y * blockDim.x + threadIdx.x; q < n; q += gridDim.y * blockDim.x) {
+        const int by = q / r.groups, kb = r.z0 + by * kBatchQuadChunk;
+        items[r.first + q] = FieldItem{r.slot, (q - by * r.groups) * kBatchQuadThreads, 0, kb,
+                                       min(kb + kBatchQuadChunk, r.z0 + r.nz) - 1, 0};
     }
 }
 
@@ -525,6 +544,8 @@ struct sgpu_batch {
     QuadInst* d_quad_inst = nullptr;
     FieldItem* d_quad[2] = {};
     size_t cap_quad[2] = {};
+    QuadRun* d_quad_run[2] = {};
+    size_t cap_quad_run[2] = {};
     bool any_quad = false, any_ring = false;  // of the listed instances
     RangeItem* d_node = nullptr;
     RangeItem* d_mnode = nullptr;  // magnetic ADE node ranges
@@ -626,7 +647,9 @@ bool running(const Slot& s, int G) { return s.ctx && G - s.start <= s.nsteps; }
 
 // Rebuild the flattened work lists from the instances that still run.
 sgpu_status rebuild(sgpu_batch* b) {
-    std::vector<FieldItem> fi[2], qi[2];
+    std::vector<FieldItem> fi[2];
+    std::vector<QuadRun> qr[2];
+    int nq[2] = {0, 0};  // quad items
     std::vector<RangeItem> node, mnode, src[2], probe, border[2];
     int nu = 1;
     b->quads_ok = b->family == 1 && !b->wait_drill;
@@ -640,9 +663,9 @@ sgpu_status rebuild(sgpu_batch* b) {
         const bool quads = b->quads_ok && b->slots[sl].quads;
         for (int side = 0; side < 2 && quads; ++side) {
             const QuadSide q = quad_side(c, side);
-            for (int kb = q.z0; kb < q.z0 + q.nz; kb += kBatchQuadChunk)
-                for (int p = 0; p < q.threads; p += kBatchQuadThreads)
-                    qi[side].push_back(FieldItem{sl, p, 0, kb, std::min(kb + kBatchQuadChunk, q.z0 + q.nz) - 1, 0});
+            const int groups = (q.threads + kBatchQuadThreads - 1) / kBatchQuadThreads;
+            qr[side].push_back(QuadRun{sl, nq[side], groups, q.z0, q.nz});
+            nq[side] += groups * ((q.nz + kBatchQuadChunk - 1) / kBatchQuadChunk);
         }
         for (int side = 0; side < 2 && !quads; ++side) {
             const int c0 = side ? 3 : 0;
@@ -687,8 +710,11 @@ sgpu_status rebuild(sgpu_batch* b) {
     sgpu_status s;
     for (int side = 0; side < 2; ++side) {
         if ((s = ensure(b, &b->d_field[side], &b->cap_field[side], fi[side].size()))) return s;
-        if ((s = ensure(b, &b->d_quad[side], &b->cap_quad[side], qi[side].size()))) return s;
-        if ((s = upload(b, b->d_quad[side], qi[side]))) return s;
+        if ((s = ensure(b, &b->d_quad[side], &b->cap_quad[side], nq[side]))) return s;
+        if ((s = ensure(b, &b->d_quad_run[side], &b->cap_quad_run[side], qr[side].size()))) return s;
+        if ((s = upload(b, b->d_quad_run[side], qr[side]))) return s;
+        if (!qr[side].empty())
+            k_quad_items<<<dim3((unsigned)qr[side].size(), 8), 256, 0, b->stream>>>(b->d_quad_run[side], b->d_quad[side]);
         if ((s = ensure(b, &b->d_src[side], &b->cap_src[side], src[side].size()))) return s;
     }
     if ((s = ensure(b, &b->d_node, &b->cap_node, node.size())) || (s = ensure(b, &b->d_probe, &b->cap_probe, probe.size())))
@@ -704,10 +730,10 @@ sgpu_status rebuild(sgpu_batch* b) {
         (s = upload(b, b->d_src[0], src[0])) || (s = upload(b, b->d_src[1], src[1])) || (s = upload(b, b->d_probe, probe)))
         return s;
     std::vector<int> counts(kNumCounts);
-    b->any_quad = !qi[0].empty();
+    b->any_quad = nq[0] > 0;
     b->any_ring = !fi[0].empty();
-    counts[kCntQuadE] = (int)qi[0].size();
-    counts[kCntQuadH] = (int)qi[1].size();
+    counts[kCntQuadE] = nq[0];
+    counts[kCntQuadH] = nq[1];
     counts[kCntE] = (int)fi[0].size();
     counts[kCntH] = (int)fi[1].size();
     counts[kCntNode] = (int)node.size();
@@ -718,6 +744,7 @@ sgpu_status rebuild(sgpu_batch* b) {
     counts[kCntMur] = (int)border[1].size();
     counts[kCntMNode] = (int)mnode.size();
     if ((s = upload(b, b->d_counts, counts))) return s;
+    BTRY(b, cudaGetLastError());
     if (nu > b->nu_max) b->nu_max = nu;
     // no wait: an asynchronous copy from pageable host memory has staged the
     // data by the time it returns, so the vectors may go out of scope, and
@@ -955,6 +982,7 @@ void sgpu_batch_destroy(sgpu_batch* b) {
     for (int s = 0; s < 2; ++s) {
         cudaFree(b->d_field[s]);
         cudaFree(b->d_quad[s]);
+        cudaFree(b->d_quad_run[s]);
         cudaFree(b->d_src[s]);
     }
     cudaFree(b->d_node);
