@@ -1254,9 +1254,6 @@ sgpu_status sgpu_batch_autotune(sgpu_batch* b, int steps_per_trial, int* chunk3,
         BTRY(b, cudaEventElapsedTime(ms, b->ev0, b->ev1));
         return check_err(b);
     };
-    bool present[kNumClasses] = {};
-    for (const Slot& sl : b->slots)
-        if (sl.ctx) present[sl.size_class] = true;
     float best = 0;
     int best_ctas = b->ctas_per_sm;
     for (int ctas : {2, 3, 4, 6}) {
@@ -1269,6 +1266,9 @@ sgpu_status sgpu_batch_autotune(sgpu_batch* b, int steps_per_trial, int* chunk3,
         }
     }
     b->ctas_per_sm = best_ctas;
+    bool present[kNumClasses] = {};  // with an instance whose items a z chunk shapes
+    for (const Slot& sl : b->slots)
+        if (sl.ctx && !(b->quads_ok && sl.quads)) present[sl.size_class] = true;
     for (int cl = 0; cl < kNumClasses; ++cl) {
         if (!present[cl]) continue;
         // longest chunks first; a shorter one must win by 3 % (fewer items

@@ -110,6 +110,21 @@ def test_autotuned_shapes_keep_results():
         _check(b, slots, pbs)
 
 
+@pytest.mark.parametrize("family", [1, 0], ids=["quads", "regs"])
+def test_autotuner_tries_only_what_shapes_the_items(family):
+    """No z chunk is tried where no instance has one: small instances in family 1."""
+    pbs = _instances()
+    with Batch(1 << 30, 16, kernel_family=family) as b:
+        b.set_tuning([7, 9, 11])
+        for pb in pbs:
+            b.add(pb)
+        chunks, _ = b.autotune(2)
+        if family == 1:
+            assert chunks == [7, 9, 11] and b.steps == 4 * 3
+        else:
+            assert chunks[0] in (8, 16, 32, 64, 128) and chunks[1:] == [9, 11] and b.steps == 9 * 3
+
+
 def test_arena_too_small_is_refused_cleanly():
     pbs = _instances()
     plan = Plan(pbs[2])
