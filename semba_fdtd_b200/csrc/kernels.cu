@@ -641,7 +641,7 @@ sgpu_status field_h(sgpu_ctx* c) {
 sgpu_status half_e(sgpu_ctx* c, StepRef sr, const StepRef* obs = nullptr) {
     sgpu_status s;
     bool sources = false;  // applied by the field kernel
-    if (c->family == 1 && quads_usable(c)) {
+    if (quads_usable(c)) {
         if ((s = ready_sources(c, 0, sr))) return s;
         if ((s = launch_quad(c, 0, sr, !c->disp_on, obs, &sources))) return s;
     } else if ((s = field_e(c))) {
@@ -654,7 +654,7 @@ sgpu_status half_e(sgpu_ctx* c, StepRef sr, const StepRef* obs = nullptr) {
 sgpu_status half_h(sgpu_ctx* c, StepRef sr, const StepRef* obs = nullptr) {
     sgpu_status s;
     bool sources = false;
-    if (c->family == 1 && quads_usable(c)) {
+    if (quads_usable(c)) {
         if ((s = ready_sources(c, 1, sr))) return s;
         if ((s = launch_quad(c, 1, sr, !c->mdisp_on, obs, &sources))) return s;
     } else if ((s = field_h(c))) {
@@ -670,14 +670,14 @@ sgpu_status half_h(sgpu_ctx* c, StepRef sr, const StepRef* obs = nullptr) {
 // that read H in the next step's E half step; the last step's follow it.
 sgpu_status whole_steps(sgpu_ctx* c, StepRef sr, int count) {
     sgpu_status s = SGPU_OK;
-    const bool ride = c->family == 1 && quads_usable(c) && observers_ride(c);
+    const bool ride = quads_usable(c) && observers_ride(c);
     for (int q = 0; q < count; ++q) {
         const StepRef now{sr.dev_n, sr.n + q}, before{sr.dev_n, sr.n + q - 1};
         if ((s = half_e(c, now, ride && q ? &before : nullptr))) return s;
         if ((s = half_h(c, now, ride ? &now : nullptr))) return s;
         if (!ride && (s = launch_probes(c, now))) return s;
     }
-    if (ride && count > 0) return launch_observe(c, 1, StepRef{sr.dev_n, sr.n + count - 1});
+    if (ride && count > 0) return launch_observe_h(c, StepRef{sr.dev_n, sr.n + count - 1});
     return SGPU_OK;
 }
 
@@ -1944,20 +1944,20 @@ sgpu_status note_probe_rows(sgpu_ctx* c, int n0, int count) {
 
 sgpu_status sgpu_advance_ex(sgpu_ctx* c) {
     SGPU_READY(c);
-    return c->family == 1 && quads_usable(c) ? launch_quad_part(c, 0, 0) : launch_e<kBulk | kCx>(c);
+    return quads_usable(c) ? launch_quad_part(c, 0, 0) : launch_e<kBulk | kCx>(c);
 }
 sgpu_status sgpu_advance_ey(sgpu_ctx* c) {
     SGPU_READY(c);
-    return c->family == 1 && quads_usable(c) ? launch_quad_part(c, 0, 1) : launch_e<kBulk | kCy>(c);
+    return quads_usable(c) ? launch_quad_part(c, 0, 1) : launch_e<kBulk | kCy>(c);
 }
 sgpu_status sgpu_advance_ez(sgpu_ctx* c) {
     SGPU_READY(c);
-    return c->family == 1 && quads_usable(c) ? launch_quad_part(c, 0, 2) : launch_e<kBulk | kCz>(c);
+    return quads_usable(c) ? launch_quad_part(c, 0, 2) : launch_e<kBulk | kCz>(c);
 }
 sgpu_status sgpu_advance_electric_cpml(sgpu_ctx* c) {
     SGPU_READY(c);
     if (!c->cpml.on) return SGPU_OK;
-    return c->family == 1 && quads_usable(c) ? launch_quad_part(c, 0, 3) : launch_e<kCpml | kAll>(c);
+    return quads_usable(c) ? launch_quad_part(c, 0, 3) : launch_e<kCpml | kAll>(c);
 }
 sgpu_status sgpu_advance_edispersive_e(sgpu_ctx* c) { SGPU_READY(c); return launch_edisp(c); }
 sgpu_status sgpu_advance_mdispersive_h(sgpu_ctx* c) { SGPU_READY(c); return launch_mdisp(c); }
@@ -1971,20 +1971,20 @@ sgpu_status sgpu_advance_nodal_e(sgpu_ctx* c, int n) {
 }
 sgpu_status sgpu_advance_hx(sgpu_ctx* c) {
     SGPU_READY(c);
-    return c->family == 1 && quads_usable(c) ? launch_quad_part(c, 1, 0) : launch_h<kBulk | kCx>(c);
+    return quads_usable(c) ? launch_quad_part(c, 1, 0) : launch_h<kBulk | kCx>(c);
 }
 sgpu_status sgpu_advance_hy(sgpu_ctx* c) {
     SGPU_READY(c);
-    return c->family == 1 && quads_usable(c) ? launch_quad_part(c, 1, 1) : launch_h<kBulk | kCy>(c);
+    return quads_usable(c) ? launch_quad_part(c, 1, 1) : launch_h<kBulk | kCy>(c);
 }
 sgpu_status sgpu_advance_hz(sgpu_ctx* c) {
     SGPU_READY(c);
-    return c->family == 1 && quads_usable(c) ? launch_quad_part(c, 1, 2) : launch_h<kBulk | kCz>(c);
+    return quads_usable(c) ? launch_quad_part(c, 1, 2) : launch_h<kBulk | kCz>(c);
 }
 sgpu_status sgpu_advance_magnetic_cpml(sgpu_ctx* c) {
     SGPU_READY(c);
     if (!c->cpml.on) return SGPU_OK;
-    return c->family == 1 && quads_usable(c) ? launch_quad_part(c, 1, 3) : launch_h<kCpml | kAll>(c);
+    return quads_usable(c) ? launch_quad_part(c, 1, 3) : launch_h<kCpml | kAll>(c);
 }
 sgpu_status sgpu_advance_planewave_h(sgpu_ctx* c, int n) {
     SGPU_READY(c);
@@ -2208,7 +2208,7 @@ sgpu_status sgpu_select_device(int device) {
 sgpu_status sgpu_kernels_per_step(const sgpu_ctx* c, int* n) {
     if (!c || !n) return SGPU_ERR_ARG;
     int k = 2;  // E and H field kernels
-    const bool quads = c->family == 1 && quads_usable(c), ride = quads && observers_ride(c);
+    const bool quads = quads_usable(c), ride = quads && observers_ride(c);
     for (const KDisp* d : {c->disp_on ? &c->disp : nullptr, c->mdisp_on ? &c->mdisp : nullptr})
         if (d) k += d->n[0] + d->n[1] + d->n[2] <= kAdeTogether ? 1 : (d->n[0] > 0) + (d->n[1] > 0) + (d->n[2] > 0);
     k += c->src[0].nrows > 0 && !(quads && !c->disp_on && rows_grouped(c, 0));

@@ -92,10 +92,10 @@ __device__ __forceinline__ void observe(const KGrid& g, const QuadObs& o, int si
     if (o.nfar && q < o.far.samples && far_step(o.far, n, m)) far_sample(g, o.far, m, side ? 2 : 1, o.ox, o.oy, o.oz, (int)q);
 }
 
-template <int SIDE>
-__global__ void __launch_bounds__(kQuadThreads) k_observe(const __grid_constant__ KGrid g, const __grid_constant__ QuadObs o) {
+// The observations of H after a call's last step, which no half step follows.
+__global__ void __launch_bounds__(kQuadThreads) k_observe_h(const __grid_constant__ KGrid g, const __grid_constant__ QuadObs o) {
     grid_wait();
-    observe(g, o, SIDE, blockIdx.x * (long long)kQuadThreads + threadIdx.x);
+    observe(g, o, 1, blockIdx.x * (long long)kQuadThreads + threadIdx.x);
 }
 
 // One half step: blocks below `blocks` march quads (bx of them a chunk of
@@ -291,7 +291,7 @@ bool quads_apart(const KCpml& cp) {
 }
 
 bool quads_usable(const sgpu_ctx* c) {
-    return tma_usable(c) && c->vol <= kQuadCells && c->quad_apart && !c->wait_drill && c->quad_mem;
+    return c->family == 1 && tma_usable(c) && c->vol <= kQuadCells && c->quad_apart && !c->wait_drill && c->quad_mem;
 }
 
 QuadView quad_view(const sgpu_ctx* c) {
@@ -447,14 +447,21 @@ static QuadObs quad_obs(const sgpu_ctx* c, int side, StepRef sr, long long* thre
     return o;
 }
 
-sgpu_status launch_observe(sgpu_ctx* c, int side, StepRef sr) {
+sgpu_status launch_observe_h(sgpu_ctx* c, StepRef sr) {
     long long threads;
-    const QuadObs o = quad_obs(c, side, sr, &threads);
+    const QuadObs o = quad_obs(c, 1, sr, &threads);
     if (threads == 0) return SGPU_OK;
     const unsigned blocks = (unsigned)((threads + kQuadThreads - 1) / kQuadThreads);
-    const cudaError_t e = side ? launch_after(c->stream, blocks, kQuadThreads, k_observe<1>, kgrid(c), o)
-                               : launch_after(c->stream, blocks, kQuadThreads, k_observe<0>, kgrid(c), o);
-    return e == cudaSuccess ? SGPU_OK : cuda_error(c, "k_observe", e);
+    const cudaError_t e = launch_after(c->stream, blocks, kQuadThreads, k_observe_h, kgrid(c), o);
+    return e == cudaSuccess ? SGPU_OK : cuda_error(c, "k_observe_h", e);
+}
+
+// Planes a thread of `bx` blocks' columns marches: fewer on grids with less than
+// 16 blocks an SM (148 of them).
+static int quad_chunk(int bx, int nz) {
+    int chunk = kQuadChunk;
+    while (chunk > 2 && (long long)bx * ((nz + chunk - 1) / chunk) < 148 * 16) chunk /= 2;
+    return chunk;
 }
 
 sgpu_status launch_quad(sgpu_ctx* c, int side, StepRef sr, bool sources, const StepRef* obs, bool* applied) {
@@ -462,8 +469,7 @@ sgpu_status launch_quad(sgpu_ctx* c, int side, StepRef sr, bool sources, const S
     if (st) return st;
     const QuadSide s = quad_side(c, side);
     const int bx = (s.threads + kQuadThreads - 1) / kQuadThreads;
-    int chunk = kQuadChunk;
-    while (chunk > 2 && (long long)bx * ((s.nz + chunk - 1) / chunk) < 148 * 16) chunk /= 2;
+    const int chunk = quad_chunk(bx, s.nz);
     const int blocks = bx * ((s.nz + chunk - 1) / chunk);
     const QuadView v = quad_view(c);
     const KGrid g = kgrid(c);
@@ -493,8 +499,7 @@ sgpu_status launch_quad(sgpu_ctx* c, int side, StepRef sr, bool sources, const S
 template <int SIDE, int MODE> static cudaError_t launch_part(sgpu_ctx* c) {
     const QuadSide s = quad_side(c, SIDE);
     const int bx = (s.threads + kQuadThreads - 1) / kQuadThreads;
-    int chunk = kQuadChunk;
-    while (chunk > 2 && (long long)bx * ((s.nz + chunk - 1) / chunk) < 148 * 16) chunk /= 2;
+    const int chunk = quad_chunk(bx, s.nz);
     return launch_after(c->stream, bx * ((s.nz + chunk - 1) / chunk), kQuadThreads, k_quad_part<SIDE, MODE>, quad_view(c), s, chunk, bx);
 }
 

@@ -389,14 +389,14 @@ void quad_alloc(sgpu_ctx* c);
 sgpu_status quad_ready(sgpu_ctx* c);
 // With `sources` the source rows of step sr are applied too when they can be
 // (*applied); with `obs` the observations of that step that read the other
-// field ride along (observers_ride).  launch_observe: those of one side alone.
+// field ride along (observers_ride).  launch_observe_h: those of H alone.
 sgpu_status launch_quad(sgpu_ctx* c, int side, StepRef sr, bool sources, const StepRef* obs, bool* applied);
 // One routine of the half step alone: components 0..2, or (3) the corrections.
 sgpu_status launch_quad_part(sgpu_ctx* c, int side, int what);
 bool rows_ride(const sgpu_ctx* c, int side);     // few enough to, where the kernels run
 bool rows_grouped(const sgpu_ctx* c, int side);  // and they do
 bool observers_ride(const sgpu_ctx* c);
-sgpu_status launch_observe(sgpu_ctx* c, int side, StepRef sr);
+sgpu_status launch_observe_h(sgpu_ctx* c, StepRef sr);
 struct FarArgs;
 FarArgs far_args(const FarField& F);
 // UpdateFarField for every far field of the context (farfield.cu).
