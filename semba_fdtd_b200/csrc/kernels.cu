@@ -552,6 +552,25 @@ void note_first_half(sgpu_ctx* c, int h) {
     c->src[0].h_first = c->src[1].h_first = h;
 }
 
+// Whether a plane wave may still act at step n or after it: pw_switch_up on the
+// host, in the same arithmetic, for the step's first half.  Once down the switch
+// stays down, so the answer for the first step of a call holds for all of them.
+bool wave_may_act(const sgpu_ctx* c, int n) {
+    bool any = false;
+    for (const auto& tb : c->src_tables) any = any || tb.is_pw;
+    if (!any) return false;
+    const int m = n - 1;  // the last step done
+    if (c->h_first < 0 || 2 * m < c->h_first || m < c->t_n0 || m >= c->t_n0 + (int)c->h_tiempo.size()) return true;
+    for (int side = 0; side < 2; ++side) {
+        const float t = (float)(c->h_tiempo[m - c->t_n0] + (side ? (double)0.5f * c->dt : 0.0));
+        bool active = false;
+        for (const auto& tb : c->src_tables)
+            active = active || (tb.is_pw && tb.has[side] && (long long)((t - tb.amax[side]) / tb.delta) + 1 <= tb.numus);
+        if (!active) return false;
+    }
+    return true;
+}
+
 // The side's source lists, and the checks of a half step at a step the host knows.
 sgpu_status ready_sources(sgpu_ctx* c, int side, StepRef sr) {
     if (c->src_dirty) {
@@ -643,7 +662,7 @@ sgpu_status half_e(sgpu_ctx* c, StepRef sr, const StepRef* obs = nullptr) {
     bool sources = false;  // applied by the field kernel
     if (quads_usable(c)) {
         if ((s = ready_sources(c, 0, sr))) return s;
-        if ((s = launch_quad(c, 0, sr, !c->disp_on, obs, &sources))) return s;
+        if ((s = launch_quad(c, 0, sr, !c->disp_on && !c->wave_up, obs, &sources))) return s;
     } else if ((s = field_e(c))) {
         return s;
     }
@@ -656,7 +675,7 @@ sgpu_status half_h(sgpu_ctx* c, StepRef sr, const StepRef* obs = nullptr) {
     bool sources = false;
     if (quads_usable(c)) {
         if ((s = ready_sources(c, 1, sr))) return s;
-        if ((s = launch_quad(c, 1, sr, !c->mdisp_on, obs, &sources))) return s;
+        if ((s = launch_quad(c, 1, sr, !c->mdisp_on && !c->wave_up, obs, &sources))) return s;
     } else if ((s = field_h(c))) {
         return s;
     }
@@ -1421,14 +1440,20 @@ sgpu_status build_sources(sgpu_ctx* c) {
         for (const SrcEntry& en : ent) k.pw_only &= en.type == kSrcPlaneWave;
         // kept wherever the quad kernels may come to serve this context: it may
         // list its rows under the wait drill and step without it
-        if (!c->arena && c->quad_mem && rows_ride(c, side)) {
-            SrcRows& h = c->src_rows[side];
-            h.first.reserve(rnode.size());
-            for (size_t r = 0; r < rnode.size(); ++r) h.first.push_back(ent[rptr[r]]);
-            h.node = std::move(rnode);
-            h.comp = std::move(rcomp);
-            h.ptr = std::move(rptr);
+        if (c->arena || !c->quad_mem) continue;
+        SrcRows rows;
+        for (size_t r = 0; r < rnode.size(); ++r) {
+            const auto b = ent.begin() + rptr[r], e = ent.begin() + rptr[r + 1];
+            if (std::all_of(b, e, [](const SrcEntry& en) { return en.type == kSrcPlaneWave; })) continue;
+            rows.node.push_back(rnode[r]);
+            rows.comp.push_back(rcomp[r]);
+            rows.start.push_back(rptr[r]);
+            rows.count.push_back((int)(e - b));
+            rows.first.push_back(*b);
         }
+        if (!rows_ride(c, side, (long long)rows.node.size())) continue;
+        rows.kept = true;
+        c->src_rows[side] = std::move(rows);
     }
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     c->src_dirty = false;
@@ -2007,8 +2032,16 @@ sgpu_status sgpu_update_observation(sgpu_ctx* c, int n) {
     return s;
 }
 
-sgpu_status sgpu_advance_e(sgpu_ctx* c, int n) { SGPU_READY(c); return half_e(c, StepRef{nullptr, n}); }
-sgpu_status sgpu_advance_h(sgpu_ctx* c, int n) { SGPU_READY(c); return half_h(c, StepRef{nullptr, n}); }
+sgpu_status sgpu_advance_e(sgpu_ctx* c, int n) {
+    SGPU_READY(c);
+    c->wave_up = wave_may_act(c, n);
+    return half_e(c, StepRef{nullptr, n});
+}
+sgpu_status sgpu_advance_h(sgpu_ctx* c, int n) {
+    SGPU_READY(c);
+    c->wave_up = wave_may_act(c, n);
+    return half_h(c, StepRef{nullptr, n});
+}
 
 sgpu_status sgpu_advance_steps(sgpu_ctx* c, int n0, int count) {
     SGPU_READY(c);
@@ -2023,9 +2056,11 @@ sgpu_status sgpu_advance_steps(sgpu_ctx* c, int n0, int count) {
     sgpu_status s = note_probe_rows(c, n0, count);
     if (s) return s;
     note_first_half(c, 2 * n0);
+    c->wave_up = wave_may_act(c, n0);
     if (quads_usable(c) && (s = quad_ready(c))) return s;
     const int chunk = std::min(count, 32);
-    if (!c->graph || c->graph_steps != chunk) {
+    const bool kept = quads_usable(c) && (c->src_rows[0].kept || c->src_rows[1].kept);
+    if (!c->graph || c->graph_steps != chunk || (kept && c->graph_wave_up != c->wave_up)) {
         if (c->graph) { cudaGraphExecDestroy(c->graph); c->graph = nullptr; }
         cudaGraph_t g;
         CUDA_TRY(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
@@ -2042,6 +2077,7 @@ sgpu_status sgpu_advance_steps(sgpu_ctx* c, int n0, int count) {
         cudaGraphDestroy(g);
         if (e != cudaSuccess) { c->graph = nullptr; return set_error(c, SGPU_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e)); }
         c->graph_steps = chunk;
+        c->graph_wave_up = c->wave_up;
     }
     k_set_step<<<1, 1, 0, c->stream>>>(c->d_step, n0);
     if ((s = check_launch(c, "k_set_step"))) return s;
@@ -2211,8 +2247,8 @@ sgpu_status sgpu_kernels_per_step(const sgpu_ctx* c, int* n) {
     const bool quads = quads_usable(c), ride = quads && observers_ride(c);
     for (const KDisp* d : {c->disp_on ? &c->disp : nullptr, c->mdisp_on ? &c->mdisp : nullptr})
         if (d) k += d->n[0] + d->n[1] + d->n[2] <= kAdeTogether ? 1 : (d->n[0] > 0) + (d->n[1] > 0) + (d->n[2] > 0);
-    k += c->src[0].nrows > 0 && !(quads && !c->disp_on && rows_grouped(c, 0));
-    k += c->src[1].nrows > 0 && !(quads && !c->mdisp_on && rows_grouped(c, 1));
+    k += c->src[0].nrows > 0 && !(quads && !c->disp_on && !c->wave_up && rows_grouped(c, 0));
+    k += c->src[1].nrows > 0 && !(quads && !c->mdisp_on && !c->wave_up && rows_grouped(c, 1));
     if (!ride) k += (c->probes.n > 0) + (int)c->vprobes.size();
     k += c->border.cl_cells > 0;
     k += c->border.mur_cells > 0;

@@ -34,7 +34,7 @@ struct QuadRow {
     int node, comp, count, first;
     SrcEntry e;
 };
-// The source rows of a half step by (warp's quads, plane), and what a row needs.
+// The nodal source rows of a half step by (warp's quads, plane), and what a row needs.
 struct QuadSrc {
     const int* ptr;  // null: none
     const QuadRow* row;
@@ -50,13 +50,20 @@ struct RowTerm {
     SrcTerm first;
     int p, end;
 };
-// Source rows ride in the half step while they are few, at most one on 25 cells:
-// a launch less (84^3 with a box inset 15, one on 43: 20.5 us a step alone,
-// against 24.5 with k_sources).  A z face of a TF/SF box puts two rows of five
-// dependent loads on each of a warp's 128 cells, so where the box fills a small
-// grid a thread a row is faster (93x41x67, one on 13: 20.7 riding, 19.0 not).
+// Nodal source rows ride in the half step, a launch less, while no plane wave acts
+// and they are at most one on 128 cells (denser was not measured).  One step alone
+// on the GPU against k_sources, spread below 1 %: 86x76x82 cells, a line of 60 nodes
+// 13.9 / 15.4 us; 170^3, a line of 128 100.8 / 103.5; 42x45x40, a plate of 64
+// 11.1 / 21.3, where k_sources also looks through 64 waveforms for a plane wave's.
+// The rows of an acting wave do not ride: where a z face of its box passes they are
+// two on each of a warp's 128 cells, with five dependent loads each, and held the
+// half step up, where k_sources has a thread a row (riding / not, 86x76x82 cells,
+// one row on 70 cells 22.4 / 17.3 us; 104^3, on 81 33.1 / 30.4; 170^3, on 84
+// 133 / 107, on 26 162 / 109).  Past, they change nothing and take no launch
+// (86x76x82 cells 13.8 us against 17.2 with k_sources, 170^3 100 / 109).
 constexpr int kRowsAtOnce = 4;
-constexpr long long kCellsARow = 25;
+constexpr long long kCellsARow = 128;
+constexpr int kNodalTerms = (1 << kSrcNodalSoft) | (1 << kSrcNodalHard);
 // Observations of one side's fields after step sr, one thread a point probe, a
 // volume probe's node or a surface sample.
 struct QuadObs {
@@ -99,7 +106,7 @@ __global__ void __launch_bounds__(kQuadThreads) k_observe_h(const __grid_constan
 }
 
 // One half step: blocks below `blocks` march quads (bx of them a chunk of
-// planes) and apply the source rows on their cells; with OBS the blocks from
+// planes) and apply the nodal source rows on their cells; with OBS the blocks from
 // there on observe the other field, which this half step leaves alone.  A step
 // is then two launches, where the sources and each kind of observation took one
 // each (84^3 with a plane wave and probes: 5 launches, 24.0 us a step alone).
@@ -126,28 +133,22 @@ __global__ void __launch_bounds__(kQuadThreads, 8)
     const int k0 = by * chunk, k1 = min(k0 + chunk, s.nz), kb = s.z0 + k0, ke = s.z0 + k1 - 1;
     for (int m = threadIdx.x; m <= ke - kb; m += kQuadThreads) zl[m] = s.z[kb + m];
     // the warp's source rows: their first contributions are formed here
-    int r0 = 0, r1 = 0, n = 0;
-    bool pw_on = false;
+    int r0 = 0, r1 = 0;
     const int lane = threadIdx.x & 31;
     if (src.ptr && p - lane < s.threads) {
         const int* sp = src.ptr + (p >> 5) * s.nz;
         r0 = sp[k0];
         r1 = sp[k1];
-        if (r0 < r1) {
-            n = step_of(src.sr);
-            pw_on = __shfl_sync(0xffffffffu, lane == 0 ? (int)pw_switch_up(src.s, n, src.tiempo, src.t_n0, src.dt, SIDE) : 0, 0) != 0;
-            if (src.s.pw_only && !pw_on) r1 = r0;
-        }
     }
-    float t = 0.0f, G21 = 0.0f;
+    float t = 0.0f;
     if (r0 < r1) {
-        const double tn = src.tiempo[n - src.t_n0];
+        const double tn = src.tiempo[step_of(src.sr) - src.t_n0];
         t = SIDE ? (float)(tn + (double)0.5f * src.dt) : (float)tn;
-        G21 = SIDE ? kg.gm2[1] : kg.g2[1];
     }
+    auto term = [&](const SrcEntry& e) { return source_term(src.s, e, t, 0.0f, kNodalTerms, false); };
     auto row_of = [&](int r) {
         const QuadRow q = src.row[r];
-        return RowTerm{kg.F[q.comp] + q.node, source_term(src.s, q.e, t, G21, 7, pw_on), q.first + 1, q.first + q.count};
+        return RowTerm{kg.F[q.comp] + q.node, term(q.e), q.first + 1, q.first + q.count};
     };
     if (r0 + lane < r1) ahead[threadIdx.x] = row_of(r0 + lane);
     int i, j;
@@ -166,7 +167,7 @@ __global__ void __launch_bounds__(kQuadThreads, 8)
         if (r0 + lane < r1) {
             const RowTerm row = ahead[threadIdx.x];
             float v = source_add(*row.f, row.first);
-            for (int e = row.p; e < row.end; ++e) v = source_add(v, source_term(src.s, src.s.e[e], t, G21, 7, pw_on));
+            for (int e = row.p; e < row.end; ++e) v = source_add(v, term(src.s.e[e]));
             *row.f = v;
         }
         for (int r = r0 + 32 + lane; r < r1; r += 32 * kRowsAtOnce) {
@@ -185,8 +186,7 @@ __global__ void __launch_bounds__(kQuadThreads, 8)
             for (int u = 0; u < kRowsAtOnce; ++u)
                 if (row[u].f) {
                     v[u] = source_add(v[u], row[u].first);
-                    for (int e = row[u].p; e < row[u].end; ++e)
-                        v[u] = source_add(v[u], source_term(src.s, src.s.e[e], t, G21, 7, pw_on));
+                    for (int e = row[u].p; e < row[u].end; ++e) v[u] = source_add(v[u], term(src.s.e[e]));
                     *row[u].f = v[u];
                 }
         }
@@ -363,10 +363,9 @@ QuadSide quad_side(const sgpu_ctx* c, int side) {
     return s;
 }
 
-// The source rows grouped by (warp's quads, plane) of their node, in the
-// kernel's numbering of the quads.  A side whose rows were not kept for this
-// (src_rows), or of which one lies on no cell the side's kernel updates, gets no
-// groups, and k_sources applies its rows.
+// The nodal source rows grouped by (warp's quads, plane) of their node, in the
+// kernel's numbering of the quads.  A side whose rows were not kept, or of which
+// one lies on no cell the side's kernel updates, gets no groups.
 static sgpu_status quad_sources(sgpu_ctx* c) {
     if (c->quad_src_ok) return SGPU_OK;
     for (void* q : c->quad_src_allocs) ctx_free(c, q);
@@ -376,7 +375,8 @@ static sgpu_status quad_sources(sgpu_ctx* c) {
         c->quad_srow[side] = nullptr;
         const SrcRows& h = c->src_rows[side];
         const size_t n = h.node.size();
-        if (n == 0 || n != (size_t)c->src[side].nrows) continue;
+        c->quad_src_all[side] = h.kept && n == 0;
+        if (n == 0) continue;
         const QuadSide s = quad_side(c, side);
         const int we = s.xlo + s.xhi, wi = s.nq - we;
         const size_t keys = (size_t)((s.threads + 31) / 32) * s.nz;
@@ -398,8 +398,7 @@ static sgpu_status quad_sources(sgpu_ctx* c) {
         for (size_t q = 0; q < keys; ++q) ptr[q + 1] += ptr[q];
         std::vector<int> at(ptr.begin(), ptr.end() - 1);
         std::vector<QuadRow> row(n);
-        for (size_t r = 0; r < n; ++r)
-            row[at[key[r]]++] = QuadRow{h.node[r], h.comp[r], h.ptr[r + 1] - h.ptr[r], h.ptr[r], h.first[r]};
+        for (size_t r = 0; r < n; ++r) row[at[key[r]]++] = QuadRow{h.node[r], h.comp[r], h.count[r], h.start[r], h.first[r]};
         int* dp = (int*)ctx_malloc(c, ptr.size() * sizeof(int));
         if (dp) c->quad_src_allocs.push_back(dp);
         void* dr = ctx_malloc(c, n * sizeof(QuadRow));
@@ -411,17 +410,18 @@ static sgpu_status quad_sources(sgpu_ctx* c) {
         if (e != cudaSuccess) return cuda_error(c, "source rows by warp", e);
         c->quad_sptr[side] = dp;
         c->quad_srow[side] = dr;
+        c->quad_src_all[side] = true;
     }
     c->quad_src_ok = true;
     return SGPU_OK;
 }
 
-bool rows_ride(const sgpu_ctx* c, int side) {
+bool rows_ride(const sgpu_ctx* c, int side, long long rows) {
     const QuadSide s = quad_side(c, side);
-    return kCellsARow * c->src[side].nrows <= 4ll * s.nq * s.ny * s.nz;
+    return kCellsARow * rows <= 4ll * s.nq * s.ny * s.nz;
 }
 
-bool rows_grouped(const sgpu_ctx* c, int side) { return c->quad_src_ok && c->quad_sptr[side]; }
+bool rows_grouped(const sgpu_ctx* c, int side) { return c->quad_src_ok && c->quad_src_all[side]; }
 
 bool observers_ride(const sgpu_ctx* c) { return (int)c->vprobes.size() <= kQuadVol && c->farfields.size() <= 1; }
 
@@ -477,7 +477,8 @@ sgpu_status launch_quad(sgpu_ctx* c, int side, StepRef sr, bool sources, const S
     if (sources && c->src[side].nrows) {
         if ((st = quad_sources(c))) return st;
         if (rows_grouped(c, side)) {
-            src = QuadSrc{c->quad_sptr[side], (const QuadRow*)c->quad_srow[side], c->src[side], c->d_tiempo, c->t_n0, c->dt, sr};
+            if (c->quad_sptr[side])
+                src = QuadSrc{c->quad_sptr[side], (const QuadRow*)c->quad_srow[side], c->src[side], c->d_tiempo, c->t_n0, c->dt, sr};
             *applied = true;
         }
     }
@@ -524,7 +525,7 @@ sgpu_status launch_quad_part(sgpu_ctx* c, int side, int what) {
 // allocation.
 sgpu_status quad_ready(sgpu_ctx* c) {
     const sgpu_status st = quad_prepare(c);
-    return st ? st : quad_sources(c);
+    return st || c->wave_up ? st : quad_sources(c);
 }
 
 }  // namespace sgpu

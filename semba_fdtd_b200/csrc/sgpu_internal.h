@@ -207,10 +207,12 @@ struct alignas(64) TMaps {
     CUtensorMap m[21];  // 9 field / media maps, then the 12 psi slabs of the side
 };
 
-// The source rows of a side on the host: node, component, where a row's
-// contributions start, and the first of them.
+// The source rows of a side that a nodal source touches, on the host: node,
+// component, a row's contributions (where they start and how many) and the first
+// of them.  Not kept where they are too many to ride.
 struct SrcRows {
-    std::vector<int> node, comp, ptr;
+    bool kept = false;
+    std::vector<int> node, comp, start, count;
     std::vector<SrcEntry> first;
 };
 
@@ -312,13 +314,18 @@ struct sgpu_ctx {
     void* quad_mem = nullptr;
     bool quad_ok = false;
     bool quad_apart = true;  // no quad of x cells meets both slabs of a CPML pair
-    // ... and a side's source rows by warp and plane (none where quad_sptr is
-    // null: the rows are k_sources' then)
+    // ... and a side's nodal source rows by warp and plane; quad_src_all: all of
+    // them (else the side's rows are k_sources')
     sgpu::SrcRows src_rows[2];
+    bool quad_src_all[2] = {};
     int* quad_sptr[2] = {};
     void* quad_srow[2] = {};
     std::vector<void*> quad_src_allocs;
     bool quad_src_ok = false;
+    // a plane wave may act in the steps being launched (set by each call that
+    // advances): the source rows are k_sources' then
+    bool wave_up = true;
+    bool graph_wave_up = true;  // as the graph was captured
     // scratch
     unsigned int* d_flag = nullptr;
     // TMA-pipelined fused kernels: tensor maps and the bounded-wait error word
@@ -387,14 +394,14 @@ bool quads_usable(const sgpu_ctx* c);
 bool quads_apart(const KCpml& cp);
 void quad_alloc(sgpu_ctx* c);
 sgpu_status quad_ready(sgpu_ctx* c);
-// With `sources` the source rows of step sr are applied too when they can be
-// (*applied); with `obs` the observations of that step that read the other
+// With `sources` (no plane wave acts) the source rows of step sr are applied too
+// when they can be (*applied); with `obs` the observations of that step that read the other
 // field ride along (observers_ride).  launch_observe_h: those of H alone.
 sgpu_status launch_quad(sgpu_ctx* c, int side, StepRef sr, bool sources, const StepRef* obs, bool* applied);
 // One routine of the half step alone: components 0..2, or (3) the corrections.
 sgpu_status launch_quad_part(sgpu_ctx* c, int side, int what);
-bool rows_ride(const sgpu_ctx* c, int side);     // few enough to, where the kernels run
-bool rows_grouped(const sgpu_ctx* c, int side);  // and they do
+bool rows_ride(const sgpu_ctx* c, int side, long long rows);  // few enough to
+bool rows_grouped(const sgpu_ctx* c, int side);               // and they can
 bool observers_ride(const sgpu_ctx* c);
 sgpu_status launch_observe_h(sgpu_ctx* c, StepRef sr);
 struct FarArgs;

@@ -1,7 +1,8 @@
 """The quad half-step kernels at the sizes where a quad can go wrong: widths
 around multiples of four and of the 32-cell pitch, CPML slabs that begin and
-end inside a quad, both sides of an axis in one quad, grids of one block and
-a few planes, and both sides of the line to the TMA ring."""
+end inside a quad, grids of one block and a few planes, and both sides of the
+line to the TMA ring; what rides in them (source rows, observations) and when
+it does not; and the contexts that they hand to other kernels."""
 import ctypes
 import tempfile
 from dataclasses import replace
@@ -77,12 +78,48 @@ def test_both_x_slabs_in_one_quad_equal_the_oracle(layers, mode):
         assert_bits_equal(got[c], o.field(c), err_msg=f"component {c}")
 
 
+def _launches(s):
+    k = ctypes.c_int()
+    s._check(s.lib.sgpu_kernels_per_step(s.handle, ctypes.byref(k)))
+    return k.value
+
+
+@pytest.mark.parametrize("mode,call", [("graph", 1), ("graph", 7), ("graph", 48), ("fused", 1)])
+def test_a_wave_that_ends(mode, call):
+    """Source rows ride in the half steps once the plane wave is past: calls of
+    one step find the first such step, longer ones begin in mid-wave.  A line of
+    36 nodes along x lies in one warp's cells, a lane more than it has."""
+    n = (41, 26, 23)
+    b = casegen._Builder(n, 150, 3)
+    b.steps([0.003], [0.003], [0.003])
+    ds = casegen.courant_dt(0.003) / 2
+    b.planewave([9] * 3, [v - 9 for v in n], 0.7, 1.9, 1.1, 0.4, "gauss.exc", ds, casegen.gaussian(ds, 20e-12, 60e-12, 0.2e-9))
+    late = casegen.gaussian_derivative(ds, 0.1e-9, 0.4e-9, 1.2e-9)
+    b.nodal([3, 12, 11], [39, 12, 11], "line.exc", ds, late)
+    b.nodal([30, 12, 11], [30, 12, 12], "dipole.exc", ds, late)
+    b.nodal([9, 10, 9], [9, 10, 14], "hard.exc", ds, late, hard=True)
+    b.probe("p", "electric", [v // 2 for v in n], "xyz")
+    pb = read_case(b.write(_DIR, "wave_ends"))
+    o = oracle.Oracle(pb)
+    want = o.step(pb.nsteps + 1)
+    seen = []
+    with Solver(pb) as s:
+        while s.n <= pb.nsteps:
+            s.step(min(call, pb.nsteps + 1 - s.n), mode=mode)
+            seen.append(_launches(s))
+        # with a step a call the probes of the fused mode have launches of their own, which are not counted
+        assert seen[0] == 4 and seen[-1] == 2 and seen == sorted(seen, reverse=True), seen
+        assert_bits_equal(s.probes(), want)
+        for c in range(6):
+            assert_bits_equal(s.field(c), o.field(c), err_msg=f"component {c}")
+
+
 @pytest.mark.parametrize("inset", [2, 5, 9])
 def test_rows_and_observers_in_the_half_steps(inset):
-    """A TF/SF box from one that fills the grid (source rows by k_sources) to a
-    small one (rows in the half step, several a lane on its z faces), with more
-    point probes than a block of observers, a volume probe of each kind and
-    field, and a step count that leaves a remainder after the captured steps."""
+    """A TF/SF box from one that fills the grid to a small one (its rows are
+    k_sources'), with more point probes than a block of observers, a volume probe
+    of each kind and field, and a step count that leaves a remainder after the
+    captured steps."""
     n = (41, 26, 23)
     b = casegen._Builder(n, 75, 3)
     b.steps([0.003], [0.003], [0.003])
@@ -121,15 +158,17 @@ def test_rows_and_observers_in_the_half_steps(inset):
                     assert_bits_equal(frames[-1][c], np.ascontiguousarray(want))
 
 
-@pytest.mark.parametrize("n", [(203, 187, 179), (301, 249, 197)])
-def test_both_sides_of_the_line_equal_the_oracle(n):
-    """Just below and just above 16 Mi padded cells, where the quads hand over
-    to the TMA ring; four steps."""
+@pytest.mark.parametrize("n,launches", [((203, 187, 179), 2), ((235, 241, 241), 2), ((235, 242, 241), 4), ((301, 249, 197), 4)])
+def test_both_sides_of_the_line_equal_the_oracle(n, launches):
+    """Below, on, just above and above the line at 16 Mi padded cells (0.52, 1, 1.004
+    and 1.07 times it), where the quads, in which the dipole and the probes ride,
+    hand over to the TMA ring; four steps."""
     pb, _ = _case(n, 6)
     pb = replace(pb, nsteps=3)
     o = oracle.Oracle(pb)
     with Solver(pb) as s:
         assert_bits_equal(s.run(), o.step(4))
+        assert _launches(s) == launches
         for c in range(6):
             assert_bits_equal(s.field(c), o.field(c), err_msg=f"component {c}")
 
@@ -227,8 +266,10 @@ def test_cpml_set_again_between_steps(kind, mode):
     b = casegen._Builder(n, 60, 5)
     b.steps([0.003], [0.003], [0.003])
     ds = casegen.courant_dt(0.003) / 2
-    b.planewave([11] * 3, [v - 11 for v in n], 0.7, 1.9, 1.1, 0.4, "gauss.exc", ds,
-                casegen.gaussian(ds, 20e-12, 60e-12, 0.2e-9))
+    wave = casegen.gaussian_derivative(ds, 20e-12, 80e-12, 0.6e-9)
+    for q in range(4):  # lines through the slabs and between them
+        b.nodal([2, 5 + 5 * q, 4 + 6 * q], [58, 5 + 5 * q, 4 + 6 * q], f"x{q}.exc", ds, wave)
+        b.nodal([7 + 13 * q, 9, 8], [7 + 13 * q, 9, 20], f"z{q}.exc", ds, wave)
     b.probe("p", "electric", [v // 2 for v in n], "xyz")
     pb = read_case(b.write(_DIR, "cpml_again"))
     out = []
@@ -238,9 +279,7 @@ def test_cpml_set_again_between_steps(kind, mode):
             _new_cpml(s, kind)
             s.step(41, mode=mode)
             out.append([s.probes()] + [s.field(c) for c in range(6)])
-            k = ctypes.c_int()
-            s._check(s.lib.sgpu_kernels_per_step(s.handle, ctypes.byref(k)))
-            assert k.value == (2 if family else 5)  # the rows ride; the probes, too, where they are the quads'
+            assert _launches(s) == (2 if family else 4)  # the rows ride, and the probes
     assert np.isfinite(out[0][1]).all() and np.abs(out[0][1]).max() > 0
     for a, w in zip(*out):
         assert_bits_equal(a, w)
