@@ -1686,6 +1686,10 @@ sgpu_status sgpu_set_time(sgpu_ctx* c, int n0, int count, const double* t) {
     c->t_n0 = n0;
     c->d_tiempo_count = count;
     c->h_tiempo.assign(t, t + count);
+    if (c->graph) {  // captured launches hold the old vector
+        cudaGraphExecDestroy(c->graph);
+        c->graph = nullptr;
+    }
     return SGPU_OK;
 }
 

@@ -348,3 +348,20 @@ def test_an_instance_without_room_for_its_tables():
         assert_bits_equal(b.probes(slot), want)
         for c in range(6):
             assert_bits_equal(b.field(slot, c), o.field(c), err_msg=f"component {c}")
+
+
+@pytest.mark.parametrize("family", [1, 0])
+def test_a_time_vector_set_between_captured_steps(family):
+    """Captured steps read the vector set last; half steps called one by one, which
+    are not captured, are the reference."""
+    pb, _ = _case((41, 26, 23), 3, steps=140)
+    out = []
+    for mode in ("graph", "fused"):
+        with Solver(pb, kernel_family=family) as s:
+            s.step(64, mode=mode)
+            t = np.ascontiguousarray(s.time_vector() * 1.25)
+            s._check(s.lib.sgpu_set_time(s.handle, 0, len(t), t.ctypes.data_as(_lib.c_double_p)), "sgpu_set_time")
+            s.step(64, mode=mode)
+            out.append([s.probes()] + [s.field(c) for c in range(6)])
+    for a, w in zip(*out):
+        assert_bits_equal(a, w)
