@@ -371,10 +371,7 @@ sgpu_status sgpu_add_farfield(sgpu_ctx* c, const sgpu_farfield_desc* d, int* id)
     }
     c->farfields.push_back(std::move(F));
     if (id) *id = (int)c->farfields.size() - 1;
-    if (c->graph) {  // the captured steps do not launch the new far field
-        cudaGraphExecDestroy(c->graph);
-        c->graph = nullptr;
-    }
+    drop_graph(c);  // the captured steps do not launch the new far field
     return SGPU_OK;
 }
 

@@ -890,7 +890,7 @@ void sgpu_destroy(sgpu_ctx* c) {
         return;
     }
     if (c->stream) cudaStreamSynchronize(c->stream);
-    if (c->graph) cudaGraphExecDestroy(c->graph);
+    drop_graph(c);
     for (int f = 0; f < 6; ++f) {
         dev_free(c, c->F[f]);
         dev_free(c, c->M[f]);
@@ -939,20 +939,14 @@ sgpu_status sgpu_synchronize(sgpu_ctx* c) {
 sgpu_status sgpu_set_wait_cycles(sgpu_ctx* c, int64_t cycles) {
     if (!c || cycles < 0) return set_error(c, SGPU_ERR_ARG, "bad wait budget");
     c->wait_cycles = cycles;
-    if (c->graph) {  // captured launches carry the old budget
-        cudaGraphExecDestroy(c->graph);
-        c->graph = nullptr;
-    }
+    drop_graph(c);  // captured launches carry the old budget
     return SGPU_OK;
 }
 
 sgpu_status sgpu_set_wait_drill(sgpu_ctx* c, int on) {
     if (!c) return SGPU_ERR_ARG;
     c->wait_drill = on ? 1 : 0;
-    if (c->graph) {
-        cudaGraphExecDestroy(c->graph);
-        c->graph = nullptr;
-    }
+    drop_graph(c);
     return SGPU_OK;
 }
 
@@ -960,10 +954,7 @@ sgpu_status sgpu_set_kernel_family(sgpu_ctx* c, int family) {
     if (!c || family < 0 || family > 1) return SGPU_ERR_ARG;
     if (family == 1 && !c->tma_ready) return set_error(c, SGPU_ERR_UNSUPPORTED, "TMA tensor maps unavailable");
     c->family = family;
-    if (c->graph) {
-        cudaGraphExecDestroy(c->graph);
-        c->graph = nullptr;
-    }
+    drop_graph(c);
     return SGPU_OK;
 }
 
@@ -1057,6 +1048,7 @@ sgpu_status sgpu_download_field(sgpu_ctx* c, int comp, float* f) {
 
 sgpu_status sgpu_init_cpml(sgpu_ctx* c, const sgpu_cpml_desc* d) {
     if (!c || !d) return set_error(c, SGPU_ERR_ARG, "null cpml descriptor");
+    drop_graph(c);  // captured launches hold the old slabs
     free_list(c, c->cpml_allocs);
     c->quad_ok = false;
     c->quad_src_ok = false;  // the slabs decide the quads' numbering
@@ -1113,16 +1105,13 @@ sgpu_status sgpu_init_cpml(sgpu_ctx* c, const sgpu_cpml_desc* d) {
                 *m = CUtensorMap{};
                 if (sl.psi && !encode_psi_map(m, sl)) c->tma_ready = false;
             }
-    if (c->graph) {
-        cudaGraphExecDestroy(c->graph);
-        c->graph = nullptr;
-    }
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     return SGPU_OK;
 }
 
 sgpu_status sgpu_init_borders(sgpu_ctx* c, const sgpu_border_desc* d) {
     if (!c || !d) return set_error(c, SGPU_ERR_ARG, "null border descriptor");
+    drop_graph(c);  // captured launches hold the old lists
     free_list(c, c->border_allocs);
     KBorder& b = c->border;
     b = KBorder{};
@@ -1195,10 +1184,6 @@ sgpu_status sgpu_init_borders(sgpu_ctx* c, const sgpu_border_desc* d) {
     }
     b.mur_cells = tot;
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-    if (c->graph) {
-        cudaGraphExecDestroy(c->graph);
-        c->graph = nullptr;
-    }
     return SGPU_OK;
 }
 
@@ -1211,6 +1196,7 @@ namespace {
 sgpu_status init_ade(sgpu_ctx* c, const sgpu_edisp_desc* d, bool mag) {
     if (!c || !d) return set_error(c, SGPU_ERR_ARG, "null pole-residue descriptor");
     if (!ready(c)) return set_error(c, SGPU_ERR_STATE, "upload the media matrices before the pole-residue set-up");
+    drop_graph(c);  // captured launches hold the old nodes
     std::vector<void*>& allocs = mag ? c->mdisp_allocs : c->disp_allocs;
     bool& on = mag ? c->mdisp_on : c->disp_on;
     const int c0 = mag ? 3 : 0;
@@ -1365,10 +1351,7 @@ long long lin(const sgpu_ctx* c, int i, int j, int k) {
 
 sgpu_status build_sources(sgpu_ctx* c) {
     c->quad_src_ok = false;
-    if (c->graph) {  // captured launches hold the old lists
-        cudaGraphExecDestroy(c->graph);
-        c->graph = nullptr;
-    }
+    drop_graph(c);  // captured launches hold the old lists
     for (int side = 0; side < 2; ++side) {
         free_list(c, c->src_allocs[side]);
         c->src[side] = KSrc{};
@@ -1686,10 +1669,7 @@ sgpu_status sgpu_set_time(sgpu_ctx* c, int n0, int count, const double* t) {
     c->t_n0 = n0;
     c->d_tiempo_count = count;
     c->h_tiempo.assign(t, t + count);
-    if (c->graph) {  // captured launches hold the old vector
-        cudaGraphExecDestroy(c->graph);
-        c->graph = nullptr;
-    }
+    drop_graph(c);  // captured launches hold the old vector
     return SGPU_OK;
 }
 
@@ -1703,6 +1683,7 @@ sgpu_status sgpu_get_time(const sgpu_ctx* c, int n0, int count, double* t) {
 
 sgpu_status sgpu_set_probes(sgpu_ctx* c, int np, const int* cijk, int cap) {
     if (!c || np < 0 || (np > 0 && (!cijk || cap <= 0))) return set_error(c, SGPU_ERR_ARG, "bad probe set");
+    drop_graph(c);  // captured launches hold the old ring
     free_list(c, c->probe_allocs);
     c->probes = KProbes{};
     c->probe_written = c->probe_read = 0;
@@ -1789,10 +1770,7 @@ sgpu_status commit_volume_probe(sgpu_ctx* c, const VolProbe& p, int* id) {
     c->vprobes.push_back(p);
     c->vprobe_read.push_back(0);
     if (id) *id = (int)c->vprobes.size() - 1;
-    if (c->graph) {  // the captured steps do not launch the new probe
-        cudaGraphExecDestroy(c->graph);
-        c->graph = nullptr;
-    }
+    drop_graph(c);  // the captured steps do not launch the new probe
     return SGPU_OK;
 }
 }  // namespace
@@ -2065,7 +2043,7 @@ sgpu_status sgpu_advance_steps(sgpu_ctx* c, int n0, int count) {
     const int chunk = std::min(count, 32);
     const bool kept = quads_usable(c) && (c->src_rows[0].kept || c->src_rows[1].kept);
     if (!c->graph || c->graph_steps != chunk || (kept && c->graph_wave_up != c->wave_up)) {
-        if (c->graph) { cudaGraphExecDestroy(c->graph); c->graph = nullptr; }
+        drop_graph(c);
         cudaGraph_t g;
         CUDA_TRY(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
         sgpu_status cs = SGPU_OK;

@@ -272,10 +272,7 @@ sgpu_status sgpu_load_resume(sgpu_ctx* c, const char* path, int* last_step) {
         // (timestepping.F90:1219): the next half step run is the first
         c->h_first = -1;
         c->src[0].h_first = c->src[1].h_first = -1;
-        if (c->graph) {
-            cudaGraphExecDestroy(c->graph);
-            c->graph = nullptr;
-        }
+        drop_graph(c);
     }
     return s;
 }

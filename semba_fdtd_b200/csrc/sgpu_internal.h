@@ -375,6 +375,12 @@ cudaError_t launch_after(cudaStream_t stream, dim3 grid, int threads, void (*ker
 #endif
 
 sgpu_status set_error(sgpu_ctx* c, sgpu_status code, const std::string& msg);
+// Captured steps hold what their launches were given; a call that frees or
+// replaces any of it drops them (cudaGraphExecDestroy leaves running ones alone).
+inline void drop_graph(sgpu_ctx* c) {
+    if (c->graph) cudaGraphExecDestroy(c->graph);
+    c->graph = nullptr;
+}
 KGrid kgrid(const sgpu_ctx* c);
 // sgpu_create with an optional arena and an external stream (batches).
 sgpu_status create_in(const sgpu_grid_desc* d, Arena* arena, cudaStream_t stream, sgpu_ctx** out);

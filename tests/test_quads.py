@@ -365,3 +365,23 @@ def test_a_time_vector_set_between_captured_steps(family):
             out.append([s.probes()] + [s.field(c) for c in range(6)])
     for a, w in zip(*out):
         assert_bits_equal(a, w)
+
+
+@pytest.mark.parametrize("family", [1, 0])
+def test_probes_set_between_captured_steps(family):
+    """Captured steps write the ring of the probes set last; half steps called one
+    by one are the reference."""
+    pb, _ = _case((41, 26, 23), 3, steps=140)
+    cijk = np.array([[0, 20, 13, 11], [5, 19, 12, 12], [1, 21, 13, 11], [2, 20, 13, 12]], np.int32)
+    out = []
+    for mode in ("graph", "fused"):
+        with Solver(pb, kernel_family=family) as s:
+            s.step(64, mode=mode)
+            first = s.probes()
+            s._check(s.lib.sgpu_set_probes(s.handle, len(cijk), cijk.ctypes.data_as(_lib.c_int_p), 64), "sgpu_set_probes")
+            s._probe_base, s._probe_rows, s.nprobes = s.n, [], len(cijk)
+            s.step(64, mode=mode)
+            out.append([first, s.probes()] + [s.field(c) for c in range(6)])
+            assert out[-1][1].shape == (64, 4)
+    for a, w in zip(*out):
+        assert_bits_equal(a, w)
