@@ -281,7 +281,12 @@ def run_ours(args):
     bytes6 = (C.c_double * 6)()
     lib.sgpu_compulsory_bytes(s.handle, bytes6)
     names = ["efield_curl_cpml", "edispersive_ade", "sources_e", "hfield_curl_cpml", "sources_h", "probes"]
-    fe, fh = ("k_tma_efield", "k_tma_hfield") if args.family == 1 else ("k_efield", "k_hfield")
+    lo = [min(a[q] for a in s.alloc) for q in (0, 2, 4)]
+    ext = [max(a[q] for a in s.alloc) - m + 1 for q, m in zip((1, 3, 5), lo)]
+    quads = (ext[0] + 31) // 32 * 32 * ext[1] * ext[2] <= 16 << 20  # padded cells, where the library takes its quad kernels
+    fe, fh, fields = (("k_efield", "k_hfield", "register-marching") if args.family == 0 else
+                      ("k_quad<0>", "k_quad<1>", "16-byte plain loads, four cells a thread") if quads else
+                      ("k_tma_efield", "k_tma_hfield", "TMA-pipelined"))
     kern = [fe, "k_ade", "k_sources", fh, "k_sources", "k_probes"]
     avg_ms = [phases[q] / K for q in range(6)]
     dom = int(np.argmax(avg_ms))
@@ -310,7 +315,7 @@ def run_ours(args):
                               if cells * 24 > 126e6 else
                               "inputs fit in L2 (fields %.0f MB); no flush between steps" % (cells * 24 / 1e6)),
                        "build": "-fmad=false (bit-exact)",
-                       "field_kernels": "TMA-pipelined" if args.family == 1 else "register-marching"},
+                       "field_kernels": fields},
             "step_roofline": {"bytes": step_bytes, "achieved": step_bytes / step_s / 1e9,
                               "frac": step_bytes / step_s / 1e9 / peak,
                               "frac_nominal": step_bytes / step_s / 1e9 / NOMINAL_HBM_GBS, "moved_bytes": step_moved,
@@ -499,7 +504,9 @@ def run_batched(args):
             "config": {"workload": CONFIGS["batched"][2], "instances": len(pbs), "cell_updates": work,
                        "arena_bytes": arena, "tuned_chunks": chunks, "tuned_ctas_per_sm": ctas,
                        "batched_arm_marks_s": marks,
-                       "field_kernels": "TMA-pipelined persistent" if args.batch_family == 1 else "register-marching"},
+                       "field_kernels": ("16-byte plain loads, four cells a thread (instances up to 16 Mi padded cells), "
+                                         "TMA-pipelined persistent (larger)"
+                                         if args.batch_family == 1 else "register-marching")},
             "plain_one_at_a_time": {"solves_per_s": len(pbs) / t_plain if not args.skip_plain else None,
                                     "seconds": None if args.skip_plain else t_plain,
                                     "gcell_upd_s": None if args.skip_plain else work / t_plain / 1e9},
@@ -550,7 +557,8 @@ def main():
     ap.add_argument("--config", default="dispersive_large", choices=list(CONFIGS))
     ap.add_argument("--n", type=int, default=None, help="scale the configuration (cells per axis)")
     ap.add_argument("--family", type=int, default=1, choices=[0, 1],
-                    help="field kernels: 1 TMA-pipelined (default), 0 register-marching")
+                    help="field kernels: 1 TMA-pipelined, or 16-byte plain loads up to 16 Mi padded cells (default), "
+                         "0 register-marching")
     ap.add_argument("--quick", action="store_true", help="skip the end-to-end and CPU-baseline legs (profiling runs)")
     ap.add_argument("--skip-cpu", action="store_true", help="skip the CPU-baseline leg and its parity check")
     ap.add_argument("--instances", type=int, default=64, help="batched: instances in the stream")
@@ -560,7 +568,8 @@ def main():
     ap.add_argument("--batch-advance-every", type=int, default=4,
                     help="batched: a 32-step chunk is queued after this many instance set-ups")
     ap.add_argument("--batch-family", type=int, default=1, choices=[0, 1],
-                    help="batched: field kernels, 1 TMA-pipelined persistent (default), 0 register-marching")
+                    help="batched: field kernels, 1 16-byte plain loads for instances up to 16 Mi padded cells and "
+                         "TMA-pipelined above (default), 0 register-marching")
     ap.add_argument("--requests", type=int, default=160, help="served: requests in the stream")
     ap.add_argument("--rate", type=float, default=32.0, help="served: Poisson arrival rate (1/s)")
     ap.add_argument("--steps-scale", type=float, default=0.25, help="served: scale of the drawn step counts")

@@ -281,10 +281,11 @@ sgpu_status sgpu_advance_e(sgpu_ctx* ctx, int n);
 sgpu_status sgpu_advance_h(sgpu_ctx* ctx, int n);
 sgpu_status sgpu_advance_steps(sgpu_ctx* ctx, int n0, int count);
 
-/* Field-kernel family of the fused half steps: 1 (default when the driver
- * provides tensor maps) streams each tile's planes through a shared-memory
- * ring with TMA bulk-tensor loads; 0 uses register-marching kernels with
- * plain loads.  Both give identical results. */
+/* Field-kernel family: 1 (default when the driver provides tensor maps) marches
+ * four x cells a thread with 16-byte plain loads on grids of up to 16 Mi padded
+ * cells, and streams larger ones tile by tile through a shared-memory ring with
+ * TMA bulk-tensor loads; 0 uses register-marching kernels with plain loads.
+ * Both give identical results. */
 sgpu_status sgpu_set_kernel_family(sgpu_ctx* ctx, int family);
 
 /* Bound, in SM clock cycles, of every wait inside the TMA-pipelined kernels
@@ -295,10 +296,10 @@ sgpu_status sgpu_set_kernel_family(sgpu_ctx* ctx, int family);
  * SGPU_ERR_TIMEOUT and the fields are then undefined.  A failure-detection
  * test shortens it to make the wait expire without a fault. */
 sgpu_status sgpu_set_wait_cycles(sgpu_ctx* ctx, int64_t cycles);
-/* Failure drill (off by default): while on, the producer warps of the
- * pipelined field kernels issue no loads, so every consumer wait runs out
- * after the wait bound and the next synchronize returns SGPU_ERR_TIMEOUT;
- * nothing is left in flight.  For tests of the timeout path. */
+/* Failure drill (off by default): while on, the pipelined field kernels serve
+ * grids of every size and their producer warps issue no loads, so every
+ * consumer wait runs out after the wait bound and the next synchronize returns
+ * SGPU_ERR_TIMEOUT; nothing is left in flight.  For tests of the timeout path. */
 sgpu_status sgpu_set_wait_drill(sgpu_ctx* ctx, int on);
 
 /* Scans the six field components for NaN/Inf on the device; returns
@@ -555,9 +556,10 @@ sgpu_status sgpu_batch_memory(sgpu_batch* b, uint64_t* capacity, uint64_t* in_us
  * buffer rounded to the arena's 256-byte grain, whole probe traces), and
  * its largest single buffer. */
 sgpu_status sgpu_batch_footprint(const sgpu_ctx* plan, uint64_t* bytes, uint64_t* largest);
-/* Field kernels of the batch: 1 (default) the persistent TMA-pipelined
- * kernels (each instance's tensor maps in global memory), 0 the
- * register-marching kernels.  Both give identical results. */
+/* Field kernels of the batch: 1 (default) 16-byte plain loads for instances up
+ * to 16 Mi padded cells and the persistent TMA-pipelined kernels above (each
+ * instance's tensor maps in global memory), 0 the register-marching kernels.
+ * Both give identical results. */
 sgpu_status sgpu_batch_set_kernel_family(sgpu_batch* b, int family);
 /* The wait bound of sgpu_set_wait_cycles for the batch's pipelined kernels;
  * sgpu_batch_synchronize reports an expiry as SGPU_ERR_TIMEOUT. */

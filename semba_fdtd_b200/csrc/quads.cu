@@ -19,12 +19,14 @@ constexpr int kQuadThreads = 64;  // 8 blocks an SM at 128 registers: 10 blocks 
 // Planes a thread marches: few, for many blocks in flight (4 against 16 planes
 // at 220^3: 191 / 207 us a step).
 constexpr int kQuadChunk = 4;
-// Up to here (padded cells) the quads are the faster half step.  Beyond, DRAM
-// streaming decides, the TMA ring's deeper prefetch catches up, and its blocks
-// leave room for another stream's.  One step of cubes with CPML 10 alone on the
-// GPU, quads against ring: 60^3 10.2 / 24.4 us, 150^3 67.8 / 91.7, 220^3
-// 191 / 209, 276^3 359 / 376, 400^3 988 / 956; 280^3 cubes of three streams
-// taking turns: 395 / 353..387.
+// Up to here (padded cells) the quads, beyond the TMA ring.  The line lies between
+// two uses: alone on the GPU the quads are the faster half step to 30 Mi and more
+// (their blocks start sooner), with three solvers taking turns on streams of their
+// own the ring is from 10 Mi on (its blocks leave room for another stream's).  A
+// step of cubes with CPML 10, quads / ring, alone (spread 2 to 4 %) and of three
+// (6 %): 8.8 Mi 155 / 170 and 147 / 148 us, 10.6 Mi 191 / 213 and 186 / 174, 15.4 Mi
+// 270 / 290 and 263 / 248, 19.9 Mi 327 / 369 and 324 / 315, 29.9 Mi 492 / 511 and
+// 493 / 458.
 constexpr long long kQuadCells = 16ll << 20;
 
 constexpr int kQuadVol = 4;  // volume probes the arguments hold

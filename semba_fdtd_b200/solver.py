@@ -290,7 +290,8 @@ class Solver:
         return out
 
     def set_kernel_family(self, family: int) -> None:
-        """1: TMA-pipelined fused field kernels (default); 0: register-marching."""
+        """1 (default): 16-byte plain loads up to 16 Mi padded cells, TMA-pipelined
+        above; 0: register-marching."""
         self._check(self.lib.sgpu_set_kernel_family(self._h, int(family)), "sgpu_set_kernel_family")
 
     # -- data --------------------------------------------------------------
