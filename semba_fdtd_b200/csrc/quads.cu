@@ -476,13 +476,12 @@ sgpu_status launch_quad(sgpu_ctx* c, int side, StepRef sr, bool sources, const S
     const QuadView v = quad_view(c);
     const KGrid g = kgrid(c);
     QuadSrc src{};
-    if (sources && c->src[side].nrows) {
-        if ((st = quad_sources(c))) return st;
-        if (rows_grouped(c, side)) {
-            if (c->quad_sptr[side])
-                src = QuadSrc{c->quad_sptr[side], (const QuadRow*)c->quad_srow[side], c->src[side], c->d_tiempo, c->t_n0, c->dt, sr};
-            *applied = true;
-        }
+    // grouped before they are needed: a later call may be under capture
+    if (c->src[side].nrows && (st = quad_sources(c))) return st;
+    if (sources && c->src[side].nrows && rows_grouped(c, side)) {
+        if (c->quad_sptr[side])
+            src = QuadSrc{c->quad_sptr[side], (const QuadRow*)c->quad_srow[side], c->src[side], c->d_tiempo, c->t_n0, c->dt, sr};
+        *applied = true;
     }
     cudaError_t e;
     long long threads = 0;
@@ -527,7 +526,7 @@ sgpu_status launch_quad_part(sgpu_ctx* c, int side, int what) {
 // allocation.
 sgpu_status quad_ready(sgpu_ctx* c) {
     const sgpu_status st = quad_prepare(c);
-    return st || c->wave_up ? st : quad_sources(c);
+    return st ? st : quad_sources(c);
 }
 
 }  // namespace sgpu
