@@ -211,9 +211,15 @@ __global__ void __launch_bounds__(kBX * kBY, 4)
 }
 
 // The half steps of small instances (quads.cuh): items are (slot, first of 64
-// quad threads in `ib`, planes kb..ke), taken in turn by resident blocks of two
-// warps.  A block holds the view of its instance in shared memory and the plane
-// lines of its item.
+// quad threads in `ib`, planes kb..ke), claimed one by one by resident blocks of
+// two warps.  A block holds the view of its instance in shared memory and the
+// plane lines of its item.
+//
+// Claimed, not dealt out by block number: with fixed shares blocks drift apart
+// over a long list until neighbouring items no longer meet in L2, and costly items
+// can fall to the same blocks.  A step, dealt / claimed (the ring at its best chunk):
+// 128 instances of 120^3 7820 / 6890 us (8610), 20 of them 1100 / 1080 (1450), 40 of
+// 168x176x60 2937 / 2264 (2577), 10 of 48^3 133 / 136 (219); spread 2 %.
 struct QuadInst {
     QuadView v;
     QuadSide s[2];
@@ -226,27 +232,40 @@ constexpr int kBatchQuadThreads = 64, kBatchQuadChunk = 8, kBatchQuadBlocks = 8;
 template <int SIDE>
 __global__ void __launch_bounds__(kBatchQuadThreads, kBatchQuadBlocks)
     k_batch_quad(const QuadInst* __restrict__ insts, const InstDesc* __restrict__ descs, const FieldItem* __restrict__ items,
-                 const int* counts, const int* G) {
+                 const int* counts, const int* G, int* next) {
     __shared__ QuadView v;
     __shared__ QuadSide s;
     __shared__ float2 tab[256];
     __shared__ QuadLine zl[kBatchQuadChunk];
-    const int n_items = counts[SIDE == 0 ? kCntQuadE : kCntQuadH];
-    int held = -1;
+    // in shared memory, not in registers, of which the march leaves none
+    __shared__ int claimed, held, n_items;
+    if (threadIdx.x == 0) {
+        held = -1;
+        n_items = counts[SIDE == 0 ? kCntQuadE : kCntQuadH];
+    }
+    __syncthreads();
     grid_wait();
-    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
+    // the other side's counter, whose kernel is done, for its next launch
+    if (blockIdx.x == 0 && threadIdx.x == 0) next[1 - SIDE] = 0;
+    for (int it = blockIdx.x; it < n_items; it = claimed) {
+        __syncthreads();  // the block is done with the last item's lines and view, and has read `claimed`
+        int more = 0;  // on its way while the item's lines are
+        if (threadIdx.x == 0) more = atomicAdd(next + SIDE, 1);
         const FieldItem w = items[it];
         bool on;
         inst_step(descs[w.slot], G, &on);
-        if (!on) continue;
-        __syncthreads();  // the block is done with the last item's lines and view
+        if (!on) {
+            if (threadIdx.x == 0) claimed = gridDim.x + more;
+            __syncthreads();
+            continue;
+        }
         if (w.slot != held) {
-            held = w.slot;
             const QuadInst& I = insts[w.slot];
             for (int q = threadIdx.x; q < (int)(sizeof(QuadView) / 4); q += kBatchQuadThreads) ((int*)&v)[q] = ((const int*)&I.v)[q];
             for (int q = threadIdx.x; q < (int)(sizeof(QuadSide) / 4); q += kBatchQuadThreads)
                 ((int*)&s)[q] = ((const int*)&I.s[SIDE])[q];
             __syncthreads();
+            if (threadIdx.x == 0) held = w.slot;
             for (int m = threadIdx.x; m < s.nmed1; m += kBatchQuadThreads) tab[m] = s.tab[m];
         }
         for (int m = threadIdx.x; m <= w.ke - w.kb; m += kBatchQuadThreads) zl[m] = s.z[w.kb + m];
@@ -257,6 +276,7 @@ __global__ void __launch_bounds__(kBatchQuadThreads, kBatchQuadBlocks)
         float idx[4];
         ld4(idx, X->id);
         const unsigned meet = valid ? X->meet & Y.hold : 0u, whole = X->whole;
+        if (threadIdx.x == 0) claimed = gridDim.x + more;
         __syncthreads();
         if (__any_sync(0xffffffffu, meet != 0)) quad_march<SIDE, true>(v, s, tab, zl, X, Y, idx, meet, whole, i, j, w.kb, w.ke, valid);
         else quad_march<SIDE, false>(v, s, tab, zl, X, Y, idx, meet, whole, i, j, w.kb, w.ke, valid);
@@ -543,6 +563,7 @@ struct sgpu_batch {
     // instances the quad kernels serve: their views by slot, and their items
     QuadInst* d_quad_inst = nullptr;
     FieldItem* d_quad[2] = {};
+    int* d_quad_next = nullptr;  // items claimed of each side's list
     size_t cap_quad[2] = {};
     QuadRun* d_quad_run[2] = {};
     size_t cap_quad_run[2] = {};
@@ -803,7 +824,7 @@ sgpu_status enqueue_step(sgpu_batch* b, cudaEvent_t* marks = nullptr) {
     const int qgrid = b->num_sms * kBatchQuadBlocks;
     if (b->any_quad)
         launch_after(b->stream, qgrid, kBatchQuadThreads, k_batch_quad<0>, b->d_quad_inst, b->d_desc, b->d_quad[0], b->d_counts,
-                     b->d_G);
+                     b->d_G, b->d_quad_next);
     if (tma && b->any_ring) {
         cudaMemsetAsync(b->d_next, 0, 2 * sizeof(int), b->stream);  // the launches' item counters
         k_batch_tma_field<0><<<tgrid, kTmaThreads, kTmaSmem, b->stream>>>(b->d_desc, b->d_maps, b->d_field[0], b->d_counts,
@@ -819,7 +840,7 @@ sgpu_status enqueue_step(sgpu_batch* b, cudaEvent_t* marks = nullptr) {
     mark(2);
     if (b->any_quad)
         launch_after(b->stream, qgrid, kBatchQuadThreads, k_batch_quad<1>, b->d_quad_inst, b->d_desc, b->d_quad[1], b->d_counts,
-                     b->d_G);
+                     b->d_G, b->d_quad_next);
     if (tma && b->any_ring)
         k_batch_tma_field<1><<<tgrid, kTmaThreads, kTmaSmem, b->stream>>>(b->d_desc, b->d_maps, b->d_field[1], b->d_counts,
                                                                           b->d_G, b->d_err, b->wait_cycles, b->wait_drill,
@@ -949,6 +970,8 @@ sgpu_status sgpu_batch_create(uint64_t arena_bytes, int max_instances, sgpu_batc
     BTRY(b, cudaMalloc((void**)&b->d_quad_inst, sizeof(QuadInst) * max_instances));
     BTRY(b, cudaMalloc((void**)&b->d_err, sizeof(int)));
     BTRY(b, cudaMalloc((void**)&b->d_next, 2 * sizeof(int)));
+    BTRY(b, cudaMalloc((void**)&b->d_quad_next, 2 * sizeof(int)));
+    BTRY(b, cudaMemsetAsync(b->d_quad_next, 0, 2 * sizeof(int), b->stream));
     BTRY(b, cudaMalloc((void**)&b->d_counts, sizeof(int) * kNumCounts));
     BTRY(b, cudaMalloc((void**)&b->d_G, sizeof(int)));
     BTRY(b, cudaMemsetAsync(b->d_err, 0, sizeof(int), b->stream));
@@ -977,6 +1000,7 @@ void sgpu_batch_destroy(sgpu_batch* b) {
     cudaFree(b->d_quad_inst);
     cudaFree(b->d_err);
     cudaFree(b->d_next);
+    cudaFree(b->d_quad_next);
     cudaFree(b->d_counts);
     cudaFree(b->d_G);
     for (int s = 0; s < 2; ++s) {

@@ -385,3 +385,19 @@ def test_probes_set_between_captured_steps(family):
             assert out[-1][1].shape == (64, 4)
     for a, w in zip(*out):
         assert_bits_equal(a, w)
+
+
+def test_a_batch_of_more_items_than_blocks():
+    """Two instances of 715 items a side, more together than the 1184 resident
+    blocks, which claim the rest; one of them finishes first, in mid-chunk, so that
+    its items do nothing for the steps left."""
+    from semba_fdtd_b200.batch import Batch
+    pb, _ = _case((110, 100, 90), 6)
+    pbs = [replace(pb, nsteps=3), replace(pb, nsteps=9)]
+    want = oracle.Oracle(pb).step(10)
+    with Batch(1 << 30, 2) as b:
+        slots = [b.add(q) for q in pbs]
+        b.advance(10)
+        b.synchronize()
+        assert_bits_equal(b.probes(slots[0]), want[:4])
+        assert_bits_equal(b.probes(slots[1]), want)
