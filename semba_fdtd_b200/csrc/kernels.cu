@@ -556,9 +556,7 @@ void note_first_half(sgpu_ctx* c, int h) {
 // host, in the same arithmetic, for the step's first half.  Once down the switch
 // stays down, so the answer for the first step of a call holds for all of them.
 bool wave_may_act(const sgpu_ctx* c, int n) {
-    bool any = false;
-    for (const auto& tb : c->src_tables) any = any || tb.is_pw;
-    if (!any) return false;
+    if (!c->has_wave) return false;
     const int m = n - 1;  // the last step done
     if (c->h_first < 0 || 2 * m < c->h_first || m < c->t_n0 || m >= c->t_n0 + (int)c->h_tiempo.size()) return true;
     for (int side = 0; side < 2; ++side) {
@@ -1337,6 +1335,7 @@ namespace {
 
 int add_table(sgpu_ctx* c, const float* ev, int numus, float delta, int is_pw) {
     sgpu_ctx::HostSrcTable t;
+    c->has_wave = c->has_wave || is_pw;
     t.samples.assign(ev, ev + numus + 1);
     t.numus = numus;
     t.delta = delta;

@@ -277,6 +277,7 @@ struct sgpu_ctx {
         float amax[2] = {0.0f, 0.0f};
     };
     std::vector<HostSrcTable> src_tables;
+    bool has_wave = false;  // one of them is a plane wave's
     struct HostEntry {
         long long node;
         int comp;
